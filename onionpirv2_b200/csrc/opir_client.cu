@@ -23,9 +23,11 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -35,6 +37,7 @@
 #include "opir_kernels.h"
 #include "opir_params.h"
 #include "opir_scan_tc.h"
+#include "opir_tc.cuh"
 
 namespace {
 
@@ -171,7 +174,9 @@ __device__ __forceinline__ uint64_t reduce_parts(const int64_t (&acc)[NP][R], in
 struct DecConst {
   uint64_t sq, t, mu_sq, mu_t;
   double inv_sq, inv_t;  // 1/sq, 1/t (wide form)
-  uint32_t wide, pad;
+  uint32_t wide;
+  uint32_t narrow;       // sq < 2^24, every dividend below 2^38, both above 2^6:
+  uint32_t m_sq, m_t;    // floor(2^38 / d) for 32-bit divisions (div_narrow)
 };
 
 // floor(x / d) for x < 2^104 whose quotient is below 2^52: the double
@@ -189,12 +194,30 @@ __device__ __forceinline__ uint64_t div_est(unsigned __int128 x, uint64_t d, dou
   return q;
 }
 
-// v mod q (canonical) for |v| < 2^104 with |v| / q below 2^52.
-__device__ __forceinline__ uint64_t mod_est(__int128 v, uint64_t q, double inv_q) {
-  const bool neg = v < 0;
-  const unsigned __int128 a = static_cast<unsigned __int128>(neg ? -v : v);
-  const uint64_t r = static_cast<uint64_t>(a - static_cast<unsigned __int128>(div_est(a, q, inv_q)) * q);
-  return neg && r ? q - r : r;
+// (lo + 2^32 hi) mod q, canonical, for |lo|, |hi| below their construction's
+// bounds: with the multiple of q (hb 2^32 + lb) added both parts are
+// nonnegative, V = hi' 2^32 + lo', and x = floor(V / 2^(32 + sh)) < 2^32.
+// m = floor(2^(64 + sh) / q): x m / 2^32 is below V / q by less than
+// 1 (m's fraction) + 2^(32 + sh) / q < 2, its floor by less than 3, so the
+// quotient estimate from one 32-bit high product leaves a remainder below 3q,
+// for which 64-bit words suffice.
+struct BigMod {
+  uint64_t q, hb, lb;
+  uint32_t m, sh;
+  __device__ __forceinline__ uint64_t operator()(int64_t lo, int64_t hi) const {
+    const uint64_t l = static_cast<uint64_t>(lo) + lb, h = static_cast<uint64_t>(hi) + hb;
+    const uint32_t x = static_cast<uint32_t>((h + (l >> 32)) >> sh);
+    uint64_t r = l + (h << 32) - __umulhi(x, m) * q;
+    r = min(r, r - 2 * q);
+    return min(r, r - q);
+  }
+};
+// floor(x / d) for x < 2^38, 2^6 < d: m = floor(2^38 / d) and x / 64 give an
+// estimate at most 2 low (x / 64's fraction, m's, the floor), corrected.
+__device__ __forceinline__ uint32_t div_narrow(uint64_t x, uint32_t d, uint32_t m) {
+  const uint32_t q = __umulhi(static_cast<uint32_t>(x >> 6), m);
+  const uint32_t r = static_cast<uint32_t>(x) - q * d;  // below 3 d
+  return q + (r >= d) + (r >= 2 * d);
 }
 
 __device__ __forceinline__ uint64_t div_barrett(uint64_t x, uint64_t d, uint64_t mu) {
@@ -232,6 +255,22 @@ __device__ __forceinline__ uint64_t decrypt_coeff(uint64_t prod, uint64_t c0, co
   return m;
 }
 
+// The same for the narrow moduli, with 32-bit divisions; prod < sq.
+__device__ __forceinline__ uint32_t decrypt_narrow(uint32_t prod, uint64_t c0, const DecConst &dc,
+                                                   uint32_t &worst) {
+  const uint32_t sq = static_cast<uint32_t>(dc.sq), t = static_cast<uint32_t>(dc.t);
+  if (c0 >= sq) c0 -= div_barrett(c0, sq, dc.mu_sq) * sq;
+  uint32_t phase = prod + static_cast<uint32_t>(c0);
+  phase = min(phase, phase - sq);
+  uint32_t m = div_narrow(static_cast<uint64_t>(phase) * t + (sq >> 1), sq, dc.m_sq);
+  m = m >= t ? m - t : m;
+  uint32_t approx = div_narrow(static_cast<uint64_t>(sq) * m + (t >> 1), t, dc.m_t);
+  approx = approx >= sq ? approx - sq : approx;
+  const uint32_t pos = phase >= approx ? phase - approx : sq - approx + phase;
+  worst = max(worst, pos > (sq >> 1) ? sq - pos : pos);
+  return m;
+}
+
 __device__ __forceinline__ void publish_noise(uint64_t worst, unsigned long long *max_noise) {
   if (!max_noise) return;
   for (int o = 16; o > 0; o >>= 1) {
@@ -244,8 +283,10 @@ __device__ __forceinline__ void publish_noise(uint64_t worst, unsigned long long
 
 // c0 of one coefficient: -(prod + e) mod q (prod = a s mod q, e any int64).
 __device__ __forceinline__ uint64_t pack_coeff(uint64_t prod, int64_t ei, uint64_t q) {
-  const uint64_t em = ei >= 0 ? static_cast<uint64_t>(ei) % q
-                              : (q - static_cast<uint64_t>(-(ei + 1)) % q - 1);
+  // |e| is a few units in practice: the 64-bit remainders only for larger ones
+  const uint64_t u = static_cast<uint64_t>(ei >= 0 ? ei : -(ei + 1));
+  const uint64_t um = u < q ? u : u % q;
+  const uint64_t em = ei >= 0 ? um : q - um - 1;
   uint64_t v = prod + em;
   if (v >= q) v -= q;
   return v ? q - v : 0;
@@ -455,12 +496,13 @@ __global__ void __launch_bounds__(kBlock) k_client_ntt(uint64_t *__restrict__ po
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) a[i] = sp[i];
 }
 
-// Tensor-core decryption (single-modulus set, small_q < 2^29): (c1 s)_i =
-// sum_j S[i][j] x_j with S[i][j] = s[i - j] (i >= j) or -s[N + i - j], so with
-// A = S + 1 (entries 0, 1, 2: one unsigned byte plane) y = A x - sum_j x_j.
-// A x mod small_q is the tensor-core scan (opir_scan_tc.h) with one residue
-// and one level: A [4 planes (1..3 zero)][N rows][N bytes], x as the four byte
-// planes of each response's c1 mod small_q, Q [4][n][N].
+// ------------------------------------------------- tensor-core product
+// (x s)_i = sum_j S[i][j] x_j with S[i][j] = s[i - j] (i >= j) or
+// -s[N + i - j], so with A = S + 1 (entries 0, 1, 2: one unsigned byte plane)
+// x s = A x - sum_j x_j, a GEMM over a batch's columns. x comes as NP byte
+// planes (3 for a 22-bit small_q, 7 for 50 bits, 8 for a ciphertext modulus),
+// so the tensor cores give S_p = A x_p exactly (int32: below 2 N 255 < 2^23)
+// and A x = sum_p 2^(8p) S_p is an exact integer; only the finish reduces.
 __global__ void __launch_bounds__(kBlock) k_client_secret_matrix(const int8_t *__restrict__ s,
                                                                  uint32_t n,
                                                                  uint8_t *__restrict__ a) {
@@ -471,151 +513,283 @@ __global__ void __launch_bounds__(kBlock) k_client_secret_matrix(const int8_t *_
   }
 }
 
-// Q planes and sum_j x_j mod small_q of response blockIdx.x.
-__global__ void __launch_bounds__(kBlock) k_client_tc_prep(const uint64_t *__restrict__ resp,
-                                                           uint32_t n, uint32_t nresp, uint64_t sq,
-                                                           uint8_t *__restrict__ qpl,
-                                                           uint64_t *__restrict__ colsum) {
-  __shared__ uint64_t part[kBlock / 32];
-  const uint64_t b = blockIdx.x;
-  const uint64_t *c1 = resp + b * 2 * n + n;
-  uint64_t sum = 0;
-  for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
-    const uint64_t x = c1[j] % sq;
-    sum += x;
+// Byte planes [NP][cols][n] of column blockIdx.x, four coefficients per
+// thread and store, and its sums of low and high 32-bit words. Column c is the
+// polynomial at x + c x_stride (reduced mod `mod` with mu = floor(2^64 / mod)
+// when mod is given), copied to copy + polynomial_of(c) when `copy` is given
+// (a query's c1 = a: query c / limbs, limb c % limbs).
+template <int NP>
+__global__ void __launch_bounds__(kBlock) k_client_planes(
+    const uint64_t *__restrict__ x, uint64_t x_stride, uint32_t n, uint32_t cols, uint64_t mod,
+    uint64_t mu, uint8_t *__restrict__ planes, uint64_t *__restrict__ colsum,
+    uint64_t *__restrict__ copy, uint32_t limbs) {
+  __shared__ uint64_t part[2][kBlock / 32];
+  const uint64_t c = blockIdx.x;
+  const uint64_t *src = x + c * x_stride;
+  uint64_t *dst = copy ? copy + ((c / limbs) * 2 * limbs + limbs + c % limbs) * n : nullptr;
+  uint64_t lo = 0, hi = 0;
+  for (uint32_t j = 4 * threadIdx.x; j < n; j += 4 * kBlock) {
+    uint64_t v[4];
 #pragma unroll
-    for (int pl = 0; pl < 4; ++pl)
-      qpl[(static_cast<uint64_t>(pl) * nresp + b) * n + j] = static_cast<uint8_t>(x >> (8 * pl));
+    for (int k = 0; k < 4; ++k) v[k] = src[j + k];
+    if (dst) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) dst[j + k] = v[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (mod) {
+        v[k] -= __umul64hi(v[k], mu) * mod;
+        v[k] = v[k] >= mod ? v[k] - mod : v[k];
+      }
+      lo += static_cast<uint32_t>(v[k]);
+      hi += v[k] >> 32;
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      uint32_t w = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) w |= static_cast<uint32_t>((v[k] >> (8 * p)) & 0xFF) << (8 * k);
+      *reinterpret_cast<uint32_t *>(planes + (static_cast<uint64_t>(p) * cols + c) * n + j) = w;
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+  for (int o = 16; o > 0; o >>= 1) {
+    lo += __shfl_xor_sync(0xFFFFFFFFu, lo, o);
+    hi += __shfl_xor_sync(0xFFFFFFFFu, hi, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    part[0][threadIdx.x >> 5] = lo;
+    part[1][threadIdx.x >> 5] = hi;
+  }
   __syncthreads();
+  if (threadIdx.x < 2) {
+    uint64_t tot = 0;
+    for (int w = 0; w < kBlock / 32; ++w) tot += part[threadIdx.x][w];
+    colsum[2 * c + threadIdx.x] = tot;
+  }
+}
+
+// The finish of one output, x s = lo + 2^32 hi of column c at coefficient i:
+// compute() is branch-free over a warp's eight columns so that their chains
+// interleave, store() follows for the columns that exist. A warp holds 32
+// adjacent coefficients of one column.
+struct FinishDecrypt {  // pt = round(phase t / sq) and the response's max noise
+  const uint64_t *resp;
+  uint64_t *pt;
+  unsigned long long *noise;
+  DecConst dc;
+  BigMod mod;     // sq (seven planes)
+  uint64_t bias;  // the multiple 2 n + 1 of sq: |x s| <= n sq
+  uint32_t n;
+  __device__ __forceinline__ uint64_t operand(uint32_t c, uint32_t i) const {
+    return __ldg(resp + static_cast<uint64_t>(c) * (2 * n) + i);
+  }
+  template <int NP>
+  __device__ __forceinline__ uint64_t compute(uint32_t, int64_t lo, int64_t hi, uint64_t c0,
+                                              uint64_t &worst) const {
+    const uint64_t v = static_cast<uint64_t>(lo) + bias;  // NP <= 4: below 2^38 (narrow), 2^43
+    if (NP == 3) {
+      const uint32_t sq = static_cast<uint32_t>(dc.sq);
+      uint32_t w = 0;
+      const uint32_t m = decrypt_narrow(static_cast<uint32_t>(v) - div_narrow(v, sq, dc.m_sq) * sq, c0, dc, w);
+      worst = w;
+      return m;
+    }
+    const uint64_t prod = NP <= 4 ? v - div_barrett(v, dc.sq, dc.mu_sq) * dc.sq : mod(lo, hi);
+    worst = 0;
+    return decrypt_coeff(prod, c0, dc, worst);
+  }
+  template <int NP>
+  __device__ __forceinline__ void store(uint32_t c, uint32_t i, uint64_t v, uint64_t worst) const {
+    pt[static_cast<uint64_t>(c) * n + i] = v;
+    if (!noise) return;
+    if (NP == 3) {
+      worst = __reduce_max_sync(0xFFFFFFFFu, static_cast<uint32_t>(worst));
+    } else {
+      for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t w = __shfl_xor_sync(0xFFFFFFFFu, worst, o);
+        worst = w > worst ? w : worst;
+      }
+    }
+    if ((threadIdx.x & 31) == 0) atomicMax(noise + c, static_cast<unsigned long long>(worst));
+  }
+};
+struct FinishPack {  // c0 = -(a s + e) mod q_limb (the constants follow)
+  const int64_t *e;
+  uint64_t *out;
+  BigMod mod[2];  // per limb
+  uint32_t n, limbs;
+  __device__ __forceinline__ uint64_t operand(uint32_t c, uint32_t i) const {
+    return static_cast<uint64_t>(__ldg(reinterpret_cast<const long long *>(e) +
+                                       static_cast<uint64_t>(limbs == 2 ? c >> 1 : c) * n + i));
+  }
+  template <int NP>
+  __device__ __forceinline__ uint64_t compute(uint32_t c, int64_t lo, int64_t hi, uint64_t ei,
+                                              uint64_t &) const {
+    const BigMod &b = mod[limbs == 2 ? c & 1 : 0];
+    return pack_coeff(b(lo, hi), static_cast<int64_t>(ei), b.q);
+  }
+  template <int NP>
+  __device__ __forceinline__ void store(uint32_t c, uint32_t i, uint64_t v, uint64_t) const {
+    const uint32_t query = limbs == 2 ? c >> 1 : c, k = limbs == 2 ? c & 1 : 0;
+    out[(static_cast<uint64_t>(query) * 2 * limbs + k) * n + i] = v;
+  }
+};
+
+struct SecretArgs {
+  uint32_t n, cols;
+  uint32_t ntile, col_tiles, k_tiles, stages;
+  const uint64_t *colsum;
+  volatile uint32_t *err;  // mapped host memory
+};
+constexpr int kSecretThreads = 64 + 256;  // producer, MMA issuer, 8 finishing warps
+constexpr uint32_t kMaxSecretStages = 8;
+
+// One CTA: one 128-row tile of A times one tile of ntile columns. Warp 0
+// streams 128-byte K slices of the A rows and of the NP planes through a ring
+// of shared-memory stages (TMA), warp 1 issues one MMA of N = NP ntile per 32
+// bytes of K (all planes of a column tile are one B operand), then eight
+// warps read the sums from TMEM, recombine and finish. A CTA takes half an
+// SM's shared memory and TMEM, so that one CTA's set-up and finish run beside
+// another's loop: at 1024 decryptions the loop and set-up take about 17 us
+// alone, the finish 13 (6 of them its DRAM traffic). All waits are bounded; a
+// wait that runs out sets the error word, and the CTA drains its copies and
+// MMAs, frees TMEM and returns.
+template <int NP, class Fin>
+__global__ void __launch_bounds__(kSecretThreads, 2)
+k_client_secret_gemm(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_x,
+                     SecretArgs a, Fin fin) {
+  using namespace opir::tc;
+  extern __shared__ __align__(1024) uint8_t sraw[];
+  uint8_t *sm = sraw + ((1024u - (sa(sraw) & 1023u)) & 1023u);
+  const uint32_t x_plane = a.ntile * 128, stage_bytes = 16384 + NP * x_plane;
+  uint64_t *full = reinterpret_cast<uint64_t *>(sm + a.stages * stage_bytes);
+  uint64_t *empty = full + kMaxSecretStages, *done = empty + kMaxSecretStages;
+  uint32_t *slot = reinterpret_cast<uint32_t *>(done + 1);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t ct = blockIdx.x % a.col_tiles, row0 = blockIdx.x / a.col_tiles * 128;
   if (threadIdx.x == 0) {
-    uint64_t t = 0;
-    for (int w = 0; w < kBlock / 32; ++w) t += part[w];
-    colsum[b] = t % sq;
-  }
-}
-
-// Two-limb decryption (small_q < 2^50): x = c1 mod small_q splits into 25-bit
-// halves; A x_half < 2 N 2^25 <= 2^38 is exact from its residues mod two
-// primes P1 P2 > 2^38 (four scans). Planes [half][4][nr][n], sums [half][nr].
-__global__ void __launch_bounds__(kBlock) k_client_tc_prep_split(const uint64_t *__restrict__ resp,
-                                                                 uint32_t n, uint32_t nr,
-                                                                 uint64_t sq,
-                                                                 uint8_t *__restrict__ qpl,
-                                                                 uint64_t *__restrict__ colsum) {
-  __shared__ uint64_t part[2][kBlock / 32];
-  const uint64_t b = blockIdx.x;
-  const uint64_t *c1 = resp + b * 2 * n + n;
-  const uint64_t plane = static_cast<uint64_t>(nr) * n;
-  uint64_t sum[2] = {0, 0};
-  for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
-    const uint64_t x = c1[j] % sq;
-    const uint64_t h[2] = {x & ((1ull << 25) - 1), x >> 25};
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      sum[hf] += h[hf];
-#pragma unroll
-      for (int pl = 0; pl < 4; ++pl)
-        qpl[(4ull * hf + pl) * plane + b * n + j] = static_cast<uint8_t>(h[hf] >> (8 * pl));
+    for (uint32_t s = 0; s < a.stages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
     }
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sa(slot)),
+                 "r"(256u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = *slot;
+  if (warp == 0) {
+    uint32_t issued = 0;
+    for (uint32_t kt = 0; kt < a.k_tiles; ++kt) {
+      const uint32_t s = kt % a.stages, ph = (kt / a.stages) & 1;
+      if (!mbar_wait(&empty[s], ph ^ 1, abort_flag)) {
+        if (lane == 0) { *abort_flag = 1; *a.err = 1u; }
+        break;
+      }
+      if (lane == 0) {
+        uint8_t *st = sm + s * stage_bytes;
+        mbar_expect_tx(&full[s], stage_bytes);
+        tma_load_3d(st, &tm_a, &full[s], kt * 128, row0, 0);
+        for (int p = 0; p < NP; ++p)
+          tma_load_3d(st + 16384 + p * x_plane, &tm_x, &full[s], kt * 128, ct * a.ntile, p);
+      }
+      __syncwarp();
+      ++issued;
+    }
+    for (uint32_t s = 0; s < a.stages; ++s) {  // copies in flight must land before the CTA exits
+      const uint32_t uses = (issued + a.stages - 1 - s) / a.stages;
+      if (uses == 0) continue;
+      const long long t0 = clock64();
+      while (!mbar_try(&full[s], (uses - 1) & 1))
+        if (clock64() - t0 > kWaitCycles) { if (lane == 0) *a.err = 8u; break; }
+    }
+  } else if (warp == 1) {
+    const uint32_t idesc = (2u << 4) | ((NP * a.ntile >> 3) << 17) | (8u << 24);  // u8 x u8 -> s32
+    for (uint32_t kt = 0; kt < a.k_tiles; ++kt) {
+      const uint32_t s = kt % a.stages, ph = (kt / a.stages) & 1;
+      if (!mbar_wait(&full[s], ph, abort_flag)) {
+        if (lane == 0) { *abort_flag = 1; *a.err = 2u; }
+        break;
+      }
+      fence_after();
+      if (lane == 0) {
+        const uint32_t base = sa(sm + s * stage_bytes);
 #pragma unroll
-  for (int hf = 0; hf < 2; ++hf) {
-    for (int o = 16; o > 0; o >>= 1) sum[hf] += __shfl_xor_sync(0xFFFFFFFFu, sum[hf], o);
-    if ((threadIdx.x & 31) == 0) part[hf][threadIdx.x >> 5] = sum[hf];
+        for (int ks = 0; ks < 4; ++ks)
+          mma_u8(tmem, smem_desc<128>(base + 32 * ks), smem_desc<128>(base + 16384 + 32 * ks), idesc, kt + ks);
+        mma_commit(&empty[s]);
+      }
+      __syncwarp();
+    }
+    if (lane == 0) mma_commit(done);
+    __syncwarp();
+    const long long t0 = clock64();
+    while (!mbar_try(done, 0))
+      if (clock64() - t0 > kWaitCycles) { if (lane == 0) *a.err = 16u; break; }
+  } else {
+    const uint32_t quad = warp & 3, part = (warp - 2) >> 2, chunks = a.ntile / 8;
+    const uint32_t i = row0 + quad * 32 + lane;
+    // a chunk is eight columns; its operands (c0 of a response, the error of
+    // a query) come from DRAM, so they are read one chunk ahead, the first
+    // under the main loop
+    const auto load = [&](uint64_t (&v)[8], uint32_t u) {
+      const uint32_t c = ct * a.ntile + 8 * u;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = u < chunks && c + k < a.cols ? fin.operand(c + k, i) : 0;
+    };
+    uint64_t next[8];
+    load(next, part);
+    const bool ok = mbar_wait(done, 0, abort_flag);
+    if (!ok && lane == 0) { *abort_flag = 1; *a.err = 4u; }
+    fence_after();
+    for (uint32_t u = part; ok && u < chunks; u += 2) {
+      const uint32_t col0 = ct * a.ntile + 8 * u;
+      uint64_t v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = next[k];
+      uint32_t S[NP][8];
+#pragma unroll
+      for (int p = 0; p < NP; ++p)
+        tmem_ld8(tmem + (quad << 21) + 8 * u + p * a.ntile, S[p]);
+      load(next, u + 2);
+      tmem_wait_ld();
+      uint64_t worst[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t c = min(col0 + k, a.cols - 1);
+        int64_t w[2];  // sums of byte planes 0..3 and 4..7, below 2^47
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (4 * h >= NP) continue;
+          uint64_t y = 0;
+#pragma unroll
+          for (int p = 3; p >= 0; --p)
+            if (4 * h + p < NP) y = (y << 8) + S[4 * h + p][k];
+          w[h] = static_cast<int64_t>(y) - static_cast<int64_t>(__ldg(a.colsum + 2ull * c + h));
+        }
+        v[k] = fin.template compute<NP>(c, w[0], NP > 4 ? w[1] : 0, v[k], worst[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (col0 + k < a.cols) fin.template store<NP>(col0 + k, i, v[k], worst[k]);  // uniform
+    }
+    fence_before();
   }
   __syncthreads();
-  if (threadIdx.x < 2) {
-    uint64_t tot = 0;
-    for (int w = 0; w < kBlock / 32; ++w) tot += part[threadIdx.x][w];
-    colsum[static_cast<uint64_t>(threadIdx.x) * nr + b] = tot;
-  }
-}
-
-// pt from the four scans ax [half][prime][nr][n]: u_half = CRT(mod P1, mod
-// P2) = A x_half exactly, y = (u_lo - sum_lo) + 2^25 (u_hi - sum_hi) = c1 s
-// (|y| < 2^62), then the decryption epilogue on y mod small_q.
-__global__ void __launch_bounds__(kBlock) k_client_tc_finish_split(
-    const uint64_t *__restrict__ resp, const uint32_t *__restrict__ ax,
-    const uint64_t *__restrict__ colsum, uint32_t n, uint32_t nr, uint64_t p1, uint64_t p2,
-    uint64_t p1_inv_mod_p2, DecConst dc, uint64_t *__restrict__ pt,
-    unsigned long long *__restrict__ max_noise) {
-  const uint64_t b = blockIdx.x;
-  const uint64_t *c0 = resp + b * 2 * n;
-  const uint64_t plane = static_cast<uint64_t>(nr) * n;
-  uint64_t worst = 0;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    int64_t y[2];
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      const uint64_t v1 = ax[(2ull * hf) * plane + b * n + i];
-      const uint64_t v2 = ax[(2ull * hf + 1) * plane + b * n + i];
-      const uint64_t v1m = v1 >= p2 ? v1 - p2 : v1;  // p1 < 2 p2
-      const uint64_t d = v2 >= v1m ? v2 - v1m : v2 + (p2 - v1m);
-      const uint64_t u = v1 + p1 * (d * p1_inv_mod_p2 % p2);
-      y[hf] = static_cast<int64_t>(u) - static_cast<int64_t>(colsum[static_cast<uint64_t>(hf) * nr + b]);
-    }
-    const int64_t v = y[0] + y[1] * (int64_t{1} << 25);
-    const int64_t r = v % static_cast<int64_t>(dc.sq);
-    const uint64_t prod = static_cast<uint64_t>(r < 0 ? r + static_cast<int64_t>(dc.sq) : r);
-    pt[b * n + i] = decrypt_coeff(prod, c0[i], dc, worst);
-  }
-  publish_noise(worst, max_noise);
-}
-
-// pt from the scan's (A x mod small_q), laid out [response][i].
-__global__ void __launch_bounds__(kBlock) k_client_tc_finish(
-    const uint64_t *__restrict__ resp, const uint32_t *__restrict__ ax,
-    const uint64_t *__restrict__ colsum, uint32_t n, DecConst dc,
-    uint64_t *__restrict__ pt, unsigned long long *__restrict__ max_noise) {
-  const uint64_t sq = dc.sq;
-  const uint64_t b = blockIdx.x;
-  const uint64_t *c0 = resp + b * 2 * n;
-  const uint64_t cs = colsum[b];
-  uint64_t worst = 0;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const uint64_t v = ax[b * n + i];
-    const uint64_t prod = v >= cs ? v - cs : v + (sq - cs);
-    pt[b * n + i] = decrypt_coeff(prod, c0[i], dc, worst);
-  }
-  publish_noise(worst, max_noise);
-}
-
-// Tensor-core packing (single-modulus set, q = q1 q2): a s mod q is the CRT
-// of a s mod q1 and mod q2, each the scan of the same A = S + 1 against the
-// byte planes of a mod q_r. Planes [r][4][nq][n], sums [r][nq].
-__global__ void __launch_bounds__(kBlock) k_client_tc_pack_prep(const uint64_t *__restrict__ a,
-                                                                uint32_t n, uint32_t nq,
-                                                                uint64_t q1, uint64_t q2,
-                                                                uint8_t *__restrict__ qpl,
-                                                                uint64_t *__restrict__ colsum) {
-  __shared__ uint64_t part[2][kBlock / 32];
-  const uint64_t b = blockIdx.x;
-  const uint64_t *x = a + b * n;
-  uint64_t sum[2] = {0, 0};
-  const uint64_t plane = static_cast<uint64_t>(nq) * n;
-  for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
-    const uint64_t r[2] = {x[j] % q1, x[j] % q2};
-#pragma unroll
-    for (int res = 0; res < 2; ++res) {
-      sum[res] += r[res];
-#pragma unroll
-      for (int pl = 0; pl < 4; ++pl)
-        qpl[(4ull * res + pl) * plane + b * n + j] = static_cast<uint8_t>(r[res] >> (8 * pl));
-    }
-  }
-#pragma unroll
-  for (int res = 0; res < 2; ++res) {
-    for (int o = 16; o > 0; o >>= 1) sum[res] += __shfl_xor_sync(0xFFFFFFFFu, sum[res], o);
-    if ((threadIdx.x & 31) == 0) part[res][threadIdx.x >> 5] = sum[res];
-  }
-  __syncthreads();
-  if (threadIdx.x < 2) {
-    uint64_t tot = 0;
-    for (int w = 0; w < kBlock / 32; ++w) tot += part[threadIdx.x][w];
-    colsum[static_cast<uint64_t>(threadIdx.x) * nq + b] = tot % (threadIdx.x ? q2 : q1);
+  if (warp == 1) {
+    fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u)
+                 : "memory");
   }
 }
 
@@ -650,125 +824,17 @@ __device__ __forceinline__ uint32_t selector_bit(const PackLayout &L, uint64_t i
   return static_cast<uint32_t>(i == 1 ? first : (perfect >> (hd - i)) & 1ull);
 }
 
-// c0 = -(a s + e) mod q plus the query's constants, c1 = a, from the two
-// scans' (A x_r mod q_r) [r][nq][n]: y_r = A x_r - sum_j x_r,j mod q_r, then
-// Garner: a s mod q = y_1 + q1 ((y_2 - y_1) q1^-1 mod q2). The constants
-// (client.cpp:128-225) are placed from the index: the one-hot at
-// BitRev(col, h), and for each set selector bit i the L_EP gadget rows at
-// BitRev(N0 + (i-1) L_EP + k, h).
-__global__ void __launch_bounds__(kBlock) k_client_tc_pack_finish(
-    const uint64_t *__restrict__ a, const int64_t *__restrict__ e,
-    const uint64_t *__restrict__ pt_idx, PackLayout L, const uint32_t *__restrict__ ax,
-    const uint64_t *__restrict__ colsum, uint32_t n, uint32_t nq, uint64_t q1, uint64_t q2,
-    uint64_t q1_inv_mod_q2, uint64_t *__restrict__ out) {
-  const uint64_t b = blockIdx.x, q = q1 * q2;
-  const uint64_t cs1 = colsum[b], cs2 = colsum[static_cast<uint64_t>(nq) + b];
-  const uint32_t *ax1 = ax + b * n, *ax2 = ax + (static_cast<uint64_t>(nq) + b) * n;
-  uint64_t *c0 = out + b * 2 * n, *c1 = c0 + n;
-  const uint64_t *x = a + b * n;
-  const int64_t *eq = e + b * n;
-  for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const uint64_t v1 = ax1[i], v2 = ax2[i];
-    const uint64_t y1 = v1 >= cs1 ? v1 - cs1 : v1 + (q1 - cs1);
-    const uint64_t y2 = v2 >= cs2 ? v2 - cs2 : v2 + (q2 - cs2);
-    const uint64_t y1m = y1 >= q2 ? y1 - q2 : y1;  // q1 < 2 q2
-    const uint64_t d = y2 >= y1m ? y2 - y1m : y2 + (q2 - y1m);
-    const uint64_t k = d * q1_inv_mod_q2 % q2;
-    c0[i] = pack_coeff(y1 + q1 * k, eq[i], q);
-    c1[i] = x[i];
-  }
-  __syncthreads();
-  const uint64_t idx = pt_idx[b];
-  const uint32_t nconst = 1 + (L.num_dims - 1) * L.l_ep;
-  for (uint32_t u = threadIdx.x; u < nconst; u += blockDim.x) {
-    uint32_t pos;
-    uint64_t val;
-    if (u == 0) {
-      pos = bitrev_dev(idx % L.n0, L.h);
-      val = L.one[0];
-    } else {
-      const uint32_t i = 1 + (u - 1) / L.l_ep, k = (u - 1) % L.l_ep;
-      if (!selector_bit(L, idx, i)) continue;
-      pos = bitrev_dev(L.n0 + static_cast<uint64_t>(i - 1) * L.l_ep + k, L.h);
-      val = L.gadget[k][0];
-    }
-    const uint64_t v = c0[pos] + val;
-    c0[pos] = v >= q ? v - q : v;
-  }
-}
-
-// Two-limb packing: every (query, limb) is one column x = a_limb mod q_limb
-// (< 2^60), split into 30-bit halves; A x_half < 2 N 2^30 <= 2^43 comes back
-// exactly from its residues mod P1 and P2. Planes [half][4][cols][n], sums
-// [half][cols], cols = queries x 2.
-__global__ void __launch_bounds__(kBlock) k_client_tc_pack_prep_split(
-    const uint64_t *__restrict__ a, uint32_t n, uint32_t cols, uint64_t q0, uint64_t q1,
-    uint8_t *__restrict__ qpl, uint64_t *__restrict__ colsum) {
-  __shared__ uint64_t part[2][kBlock / 32];
-  const uint64_t col = blockIdx.x;
-  const uint64_t q = (col & 1) ? q1 : q0;
-  const uint64_t *x = a + col * n;
-  const uint64_t plane = static_cast<uint64_t>(cols) * n;
-  uint64_t sum[2] = {0, 0};
-  for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
-    const uint64_t v = x[j] % q;
-    const uint64_t h[2] = {v & ((1ull << 30) - 1), v >> 30};
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      sum[hf] += h[hf];
-#pragma unroll
-      for (int pl = 0; pl < 4; ++pl)
-        qpl[(4ull * hf + pl) * plane + col * n + j] = static_cast<uint8_t>(h[hf] >> (8 * pl));
-    }
-  }
-#pragma unroll
-  for (int hf = 0; hf < 2; ++hf) {
-    for (int o = 16; o > 0; o >>= 1) sum[hf] += __shfl_xor_sync(0xFFFFFFFFu, sum[hf], o);
-    if ((threadIdx.x & 31) == 0) part[hf][threadIdx.x >> 5] = sum[hf];
-  }
-  __syncthreads();
-  if (threadIdx.x < 2) {
-    uint64_t tot = 0;
-    for (int w = 0; w < kBlock / 32; ++w) tot += part[threadIdx.x][w];
-    colsum[static_cast<uint64_t>(threadIdx.x) * cols + col] = tot;
-  }
-}
-
-// Query blockIdx.x: per limb k, a_k s = (A x_lo - sum_lo) + 2^30 (A x_hi -
-// sum_hi) (|.| < 2^73, 128-bit) mod q_k, c0 = -(a_k s + e) plus the constants
-// placed from the index, c1 = a.
-__global__ void __launch_bounds__(kBlock) k_client_tc_pack_finish_split(
-    const uint64_t *__restrict__ a, const int64_t *__restrict__ e,
-    const uint64_t *__restrict__ pt_idx, PackLayout L, const uint32_t *__restrict__ ax,
-    const uint64_t *__restrict__ colsum, uint32_t n, uint32_t cols, uint64_t p1, uint64_t p2,
-    uint64_t p1_inv_mod_p2, uint64_t q0, uint64_t q1, double inv_q0, double inv_q1,
-    uint64_t *__restrict__ out) {
+// Adds query blockIdx.x's constants (client.cpp:128-225) to its c0 from the
+// index: the one-hot at BitRev(col, h), and for each set selector bit i the
+// L_EP gadget rows at BitRev(N0 + (i-1) L_EP + k, h), per limb.
+__global__ void __launch_bounds__(128) k_client_pack_constants(
+    const uint64_t *__restrict__ pt_idx, PackLayout L, uint32_t n, uint32_t limbs, uint64_t q0,
+    uint64_t q1, uint64_t *__restrict__ out) {
   const uint64_t b = blockIdx.x;
-  const uint64_t plane = static_cast<uint64_t>(cols) * n;
-  uint64_t *c0 = out + b * 4 * n, *c1 = c0 + 2 * n;
-  const int64_t *eq = e + b * n;
-  for (uint32_t w = threadIdx.x; w < 2 * n; w += blockDim.x) {
-    const uint32_t k = w / n, i = w % n;
-    const uint64_t col = 2 * b + k, q = k ? q1 : q0;
-    __int128 y[2];
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      const uint64_t v1 = ax[(2ull * hf) * plane + col * n + i];
-      const uint64_t v2 = ax[(2ull * hf + 1) * plane + col * n + i];
-      const uint64_t v1m = v1 >= p2 ? v1 - p2 : v1;
-      const uint64_t d = v2 >= v1m ? v2 - v1m : v2 + (p2 - v1m);
-      const uint64_t u = v1 + p1 * (d * p1_inv_mod_p2 % p2);
-      y[hf] = static_cast<__int128>(u) - static_cast<__int128>(colsum[static_cast<uint64_t>(hf) * cols + col]);
-    }
-    const uint64_t v = mod_est(y[0] + y[1] * (static_cast<__int128>(1) << 30), q,
-                               k ? inv_q1 : inv_q0);
-    c0[w] = pack_coeff(v, eq[i], q);
-    c1[w] = a[col * n + i];
-  }
-  __syncthreads();
+  uint64_t *c0 = out + b * 2 * limbs * n;
   const uint64_t idx = pt_idx[b];
   const uint32_t nconst = 1 + (L.num_dims - 1) * L.l_ep;
-  for (uint32_t u = threadIdx.x; u < 2 * nconst; u += blockDim.x) {
+  for (uint32_t u = threadIdx.x; u < limbs * nconst; u += blockDim.x) {
     const uint32_t k = u / nconst, cu = u % nconst;
     const uint64_t q = k ? q1 : q0;
     uint32_t pos;
@@ -783,8 +849,8 @@ __global__ void __launch_bounds__(kBlock) k_client_tc_pack_finish_split(
       val = L.gadget[r][k];
     }
     uint64_t *cell = c0 + static_cast<uint64_t>(k) * n + pos;
-    const uint64_t s2 = *cell + val;
-    *cell = s2 >= q ? s2 - q : s2;
+    const uint64_t v = *cell + val;
+    *cell = v >= q ? v - q : v;
   }
 }
 
@@ -797,6 +863,62 @@ uint64_t bitrev(uint64_t x, uint32_t bits) {
 
 uint64_t mulmod(uint64_t a, uint64_t b, uint64_t m) {
   return static_cast<uint64_t>(static_cast<unsigned __int128>(a) * b % m);
+}
+
+}  // namespace
+
+namespace {
+
+// Error words of the tensor-core product in one mapped page of pinned host
+// memory per process (the kernels write a word only when a bounded wait runs
+// out, so reading it takes no copy). Pinning memory takes about a millisecond,
+// more than a whole batch, hence one page for all handles: a handle takes a
+// word at its first product and gives it back when it is destroyed, the page
+// goes with the last one. Handles beyond the page's words pin their own.
+class ErrorWords {
+ public:
+  uint32_t *take() {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (!page_) {
+      page_ = pin(kWords);
+      for (uint32_t i = kWords; i-- > 0;) free_.push_back(page_ + i);
+    }
+    if (free_.empty()) return pin(1);
+    uint32_t *w = free_.back();
+    free_.pop_back();
+    *w = 0;
+    return w;
+  }
+  void give_back(uint32_t *w) {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (!page_ || w < page_ || w >= page_ + kWords) {
+      cudaFreeHost(w);
+      return;
+    }
+    free_.push_back(w);
+    if (free_.size() == kWords) {
+      free_.clear();
+      cudaFreeHost(page_);
+      page_ = nullptr;
+    }
+  }
+
+ private:
+  static constexpr uint32_t kWords = 1024;
+  static uint32_t *pin(uint32_t words) {
+    void *p = nullptr;
+    ck(cudaHostAlloc(&p, words * sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable),
+       "client error word");
+    std::memset(p, 0, words * sizeof(uint32_t));
+    return static_cast<uint32_t *>(p);
+  }
+  std::mutex mu_;
+  uint32_t *page_ = nullptr;
+  std::vector<uint32_t *> free_;
+};
+ErrorWords &error_words() {
+  static ErrorWords *w = new ErrorWords;  // never destroyed: handles may outlive static objects
+  return *w;
 }
 
 }  // namespace
@@ -815,9 +937,8 @@ struct opir_client {
   DevBuf<KeyRow> keyrows;
   // tensor-core decryption: A = S + 1 (built on first use), per-call scratch
   DevBuf<uint8_t> tc_a, tc_q;
-  DevBuf<uint64_t> tc_colsum, pk_colsum;
-  DevBuf<uint32_t> tc_ax, tc_err, pk_ax;
-  DevBuf<uint8_t> pk_q;
+  DevBuf<uint64_t> tc_colsum;
+  uint32_t *tc_err = nullptr;        // error word of the product (ErrorWords)
   DevBuf<uint64_t> pk_idx;
   uint64_t *idx_staging = nullptr;   // pinned copy of the last call's indices
   size_t idx_staging_cap = 0;
@@ -1053,10 +1174,36 @@ DecConst dec_const(const opir_params &p) {
   dc.wide = static_cast<unsigned __int128>(dc.sq) * dc.t + dc.sq >= (static_cast<unsigned __int128>(1) << 63);
   dc.inv_sq = 1.0 / static_cast<double>(dc.sq);
   dc.inv_t = 1.0 / static_cast<double>(dc.t);
+  dc.narrow = dc.sq < (1ull << 24) && dc.sq > 64 && dc.t > 64 && dc.t < (1ull << 24) &&
+              dc.sq * (dc.t + 1) < (1ull << 38) && dc.sq * (3ull * p.poly_degree + 1) < (1ull << 38);
+  if (dc.narrow) {
+    dc.m_sq = static_cast<uint32_t>((1ull << 38) / dc.sq);
+    dc.m_t = static_cast<uint32_t>((1ull << 38) / dc.t);
+  }
   return dc;
 }
 
-// The tensor-core form serves single-modulus decryption batches of at least
+// Reduction of lo + 2^32 hi with |lo| <= 2 n 2^lo_bits, |hi| <= 2 n 2^hi_bits.
+BigMod big_mod(uint64_t q, uint32_t n, uint32_t lo_bits, uint32_t hi_bits) {
+  uint32_t ln = 1;  // 2 n <= 2^ln
+  while ((1ull << ln) < 2ull * n) ++ln;
+  using u128 = unsigned __int128;
+  BigMod b{};
+  b.q = q;
+  // hi' + lo' / 2^32 < 2^(hi_bits + ln + 2) + 2^(lo_bits + ln + 2 - 32)
+  const uint32_t top = std::max(hi_bits + ln + 3, lo_bits + ln + 3 > 32 ? lo_bits + ln + 3 - 32 : 1);
+  b.sh = top > 32 ? top - 32 : 0;
+  b.m = static_cast<uint32_t>((static_cast<u128>(1) << (64 + b.sh)) / q);
+  // the least multiple of q at or above the magnitude of both parts, split
+  // with lb >= 2 n 2^lo_bits
+  const u128 need = (static_cast<u128>(1) << (hi_bits + ln + 32)) + (static_cast<u128>(1) << (lo_bits + ln + 1));
+  const u128 bias = (need + q - 1) / q * q;
+  b.lb = static_cast<uint64_t>(bias & 0xFFFFFFFFu) + (1ull << std::max<uint32_t>(lo_bits + ln, 32));
+  b.hb = static_cast<uint64_t>((bias - b.lb) >> 32);
+  return b;
+}
+
+// The tensor-core form serves decryption and packing batches of at least
 // kTcMinResponses (OPIR_CLIENT_TC=0 turns it off).
 constexpr uint64_t kTcMinResponses = 32;
 // any_limbs: decryption, whose modulus (small_q) is one prime for both sets.
@@ -1071,71 +1218,86 @@ bool tc_enabled(const opir_client &c, uint64_t items, uint64_t modulus_bound,
 void ensure_secret_matrix(opir_client &c, cudaStream_t st) {
   if (c.tc_a.p) return;
   const uint32_t n = c.n;
-  c.tc_a.alloc(4ull * n * n);
-  ck(cudaMemsetAsync(c.tc_a.p, 0, 4ull * n * n, st), "secret matrix clear");
-  k_client_secret_matrix<<<n, kBlock, 0, st>>>(c.msgs.p, n, c.tc_a.p);
+  opir::DevBuf<uint8_t> a;
+  a.alloc(static_cast<size_t>(n) * n);
+  if (!c.tc_err) c.tc_err = error_words().take();
+  k_client_secret_matrix<<<n, kBlock, 0, st>>>(c.msgs.p, n, a.p);
   launched("secret matrix launch");
-  c.tc_err.alloc(1);
+  std::swap(c.tc_a.p, a.p);
+  std::swap(c.tc_a.n, a.n);
 }
 
-// One scan C = A x mod q (< 2^29) over nr columns of byte planes `planes`
-// ([4][nr][n]) into cmat [nr][n].
-void scan_secret_matrix(const opir_client &c, uint32_t nr, uint64_t q, const uint8_t *planes,
-                        uint32_t *cmat, cudaStream_t st) {
+// Columns per tile of the secret product (16, 32 or 64, NP ntile <= 256): the
+// largest that leaves one and a half CTAs per SM (an SM holds two), since a
+// larger tile reads A fewer times, else the smallest. At 1024 decryptions
+// (N = 2048) 64 columns give 256 CTAs and 30 us, 32 give 512 and 33 us; at
+// 777 packings 32 columns give 400 CTAs and 46 us.
+uint32_t secret_ntile(uint32_t np, uint32_t n, uint64_t cols, int sms) {
+  for (uint32_t nt : {64u, 32u})
+    if (np * nt <= 256 && n / 128 * ((cols + nt - 1) / nt) >= 3ull * sms / 2) return nt;
+  return 16;
+}
+
+// planes [NP][cols][n] and colsum as k_client_planes writes them
+template <int NP, class Fin>
+void secret_product(const opir_client &c, uint64_t cols, const uint8_t *planes,
+                    const uint64_t *colsum, const Fin &fin, cudaStream_t st) {
+  constexpr size_t kLimit = 113 * 1024;  // half an SM
   const uint32_t n = c.n;
-  opir::TcScanArgs a{};
-  a.ntile = nr <= 16 ? 16 : nr <= 32 ? 32 : 64;
-  a.kt = 128;
-  a.stages = opir::scan_tc_max_stages(a.ntile, a.kt);
-  a.col_tiles = (nr + a.ntile - 1) / a.ntile;
-  a.k_tiles = n / a.kt;
-  a.other = n;
-  a.m_tiles = n / 128;
-  a.ncols = nr;
-  a.zcount = 1;
-  a.levels_per_res = 1;
-  a.q[0] = a.q[1] = static_cast<uint32_t>(q);
-  a.mu[0] = a.mu[1] = static_cast<uint64_t>((static_cast<unsigned __int128>(1) << 64) / q);
-  uint64_t w = 1;
-  for (int sft = 0; sft < 7; ++sft) {
-    a.w[0][sft] = a.w[1][sft] = static_cast<uint32_t>(w);
-    w = (w << 8) % q;
-  }
-  a.cmat = cmat;
-  a.err = c.tc_err.p;
-  CUtensorMap map_a, map_q;
-  opir::make_plane_map(&map_a, c.tc_a.p, n, n, 4, 128, 128);
-  opir::make_plane_map(&map_q, planes, n, nr, 4, a.ntile, 128);
-  opir::launch_scan_tc(map_a, map_q, a, c.sms, st);
+  SecretArgs a{};
+  a.n = n;
+  a.cols = static_cast<uint32_t>(cols);
+  a.ntile = secret_ntile(NP, n, cols, c.sms);
+  a.col_tiles = static_cast<uint32_t>((cols + a.ntile - 1) / a.ntile);
+  a.k_tiles = n / 128;
+  const size_t stage = 16384 + NP * a.ntile * 128;
+  a.stages = static_cast<uint32_t>(std::min<size_t>(kMaxSecretStages, (kLimit - 1024 - 256) / stage));
+  a.colsum = colsum;
+  void *err = nullptr;
+  ck(cudaHostGetDevicePointer(&err, c.tc_err, 0), "client error word");
+  a.err = static_cast<volatile uint32_t *>(err);
+  CUtensorMap map_a, map_x;
+  opir::make_plane_map(&map_a, c.tc_a.p, n, n, 1, 128, 128);
+  opir::make_plane_map(&map_x, planes, n, cols, NP, a.ntile, 128);
+  auto kern = k_client_secret_gemm<NP, Fin>;
+  ck(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kLimit)),
+     "cudaFuncSetAttribute");
+  kern<<<a.col_tiles * (n / 128), kSecretThreads, 1024 + a.stages * stage + 256, st>>>(map_a, map_x,
+                                                                                      a, fin);
+  launched("client secret product launch");
 }
 
-// Reads the scans' error word (synchronises the stream).
-void check_scan_error(const opir_client &c, cudaStream_t st, const char *what) {
-  uint32_t err = 0;
-  ck(cudaMemcpyAsync(&err, c.tc_err.p, sizeof(err), cudaMemcpyDeviceToHost, st), "scan error read");
+// Synchronises the stream and reads the products' error word, which lies in
+// mapped host memory: the kernels write it only when a bounded wait runs out.
+void check_product_error(opir_client &c, cudaStream_t st, const char *what) {
   ck(cudaStreamSynchronize(st), what);
-  if (err) throw std::runtime_error(std::string(what) + ": tensor-core scan gave up (error bits " +
-                                    std::to_string(err) + ")");
+  const uint32_t err = *const_cast<volatile uint32_t *>(c.tc_err);
+  if (err) {
+    *c.tc_err = 0;
+    throw std::runtime_error(std::string(what) + ": tensor-core product gave up (error bits " +
+                             std::to_string(err) + ")");
+  }
 }
 
-// The two primes of the split forms (29-bit, product above 2^57).
-constexpr uint64_t kSplitP1 = 536813569, kSplitP2 = 536752129;
+// Byte planes and column sums for `cols` columns of np planes.
+void ensure_planes(opir_client &c, uint32_t np, uint64_t cols, cudaStream_t st) {
+  const uint64_t bytes = static_cast<uint64_t>(np) * cols * c.n;
+  if (c.tc_q.n >= bytes && c.tc_colsum.n >= 2 * cols) return;
+  ck(cudaStreamSynchronize(st), "client sync");
+  if (c.tc_q.n < bytes) c.tc_q.alloc(bytes);
+  if (c.tc_colsum.n < 2 * cols) c.tc_colsum.alloc(2 * cols);
+}
 
 void launch_pack_tc(uint64_t n_q, const uint64_t *pt_idx, cudaStream_t st, const uint64_t *a,
                     const int64_t *e, opir_client &c, uint64_t *out) {
-  const uint32_t n = c.n, nq = static_cast<uint32_t>(n_q);
+  const uint32_t n = c.n, limbs = c.limbs;
   const opir_params &p = c.params;
   if (p.l_ep > 16) throw std::runtime_error("client pack: L_EP above 16");
   ensure_secret_matrix(c, st);
-  // columns: one per query (single modulus: two residue sets) or one per
-  // (query, limb) (two limbs: two 30-bit halves); both need 8 plane sets'
-  // worth of room per column pair
-  const uint64_t cols = n_q * c.limbs;
-  if (c.pk_colsum.n < 2 * cols) {
+  const uint64_t cols = n_q * limbs;  // one column per query and limb
+  ensure_planes(c, 8, cols, st);
+  if (c.pk_idx.n < n_q) {
     ck(cudaStreamSynchronize(st), "client sync");
-    c.pk_q.alloc(8ull * cols * n);
-    c.pk_colsum.alloc(2 * cols);
-    c.pk_ax.alloc((c.limbs == 2 ? 4 : 2) * cols * n);
     c.pk_idx.alloc(n_q);
   }
   // the previous call's index upload must have left the staging buffer
@@ -1163,88 +1325,50 @@ void launch_pack_tc(uint64_t n_q, const uint64_t *pt_idx, cudaStream_t st, const
     L.gadget[k][0] = c.gadget_val[2 * k];
     L.gadget[k][1] = c.gadget_val[2 * k + 1];
   }
-  ck(cudaMemsetAsync(c.tc_err.p, 0, sizeof(uint32_t), st), "scan error reset");
-  if (c.limbs == 2) {
-    const uint32_t nc = static_cast<uint32_t>(cols);
-    uint64_t inv = 0;
-    if (!opir::invert_mod(kSplitP1 % kSplitP2, kSplitP2, inv)) throw std::runtime_error("split primes");
-    k_client_tc_pack_prep_split<<<nc, kBlock, 0, st>>>(a, n, nc, p.q1, p.q2, c.pk_q.p,
-                                                       c.pk_colsum.p);
-    launched("client pack prep launch");
-    const uint64_t set = 4ull * cols * n, outw = cols * n;
-    for (int hf = 0; hf < 2; ++hf)
-      for (int pr = 0; pr < 2; ++pr)
-        scan_secret_matrix(c, nc, pr ? kSplitP2 : kSplitP1, c.pk_q.p + hf * set,
-                           c.pk_ax.p + (2 * hf + pr) * outw, st);
-    k_client_tc_pack_finish_split<<<nq, kBlock, 0, st>>>(a, e, c.pk_idx.p, L, c.pk_ax.p,
-                                                         c.pk_colsum.p, n, nc, kSplitP1, kSplitP2,
-                                                         inv, p.q1, p.q2, 1.0 / static_cast<double>(p.q1),
-                                                         1.0 / static_cast<double>(p.q2), out);
-    launched("client pack finish launch");
-    check_scan_error(c, st, "client pack");
-    return;
-  }
-  k_client_tc_pack_prep<<<nq, kBlock, 0, st>>>(a, n, nq, p.q1, p.q2, c.pk_q.p, c.pk_colsum.p);
-  launched("client pack prep launch");
-  const uint64_t plane_set = 4ull * n_q * n;
-  scan_secret_matrix(c, nq, p.q1, c.pk_q.p, c.pk_ax.p, st);
-  scan_secret_matrix(c, nq, p.q2, c.pk_q.p + plane_set, c.pk_ax.p + n_q * n, st);
-  k_client_tc_pack_finish<<<nq, kBlock, 0, st>>>(a, e, c.pk_idx.p, L, c.pk_ax.p,
-                                                 c.pk_colsum.p, n, nq, p.q1, p.q2,
-                                                 p.q1_inv_mod_q2, out);
-  launched("client pack finish launch");
-  check_scan_error(c, st, "client pack");
+  k_client_planes<8><<<static_cast<unsigned>(cols), kBlock, 0, st>>>(
+      a, n, n, static_cast<uint32_t>(cols), 0, 0, c.tc_q.p, c.tc_colsum.p, out, limbs);
+  launched("client planes launch");
+  FinishPack fin{};
+  fin.e = e;
+  fin.out = out;
+  fin.n = n;
+  fin.limbs = limbs;
+  // words of any 64-bit a: both halves below 2^32
+  for (uint32_t k = 0; k < limbs; ++k) fin.mod[k] = big_mod(c.mods[k], n, 32, 32);
+  secret_product<8>(c, cols, c.tc_q.p, c.tc_colsum.p, fin, st);
+  k_client_pack_constants<<<static_cast<unsigned>(n_q), 128, 0, st>>>(c.pk_idx.p, L, n, limbs,
+                                                                     c.mods[0], c.mods[1], out);
+  launched("client constants launch");
+  check_product_error(c, st, "client pack");
 }
 
-void launch_decrypt_tc_split(uint64_t n_resp, cudaStream_t st, const uint64_t *resp,
-                             opir_client &c, uint64_t *pt, unsigned long long *noise) {
-  const uint32_t n = c.n, nr = static_cast<uint32_t>(n_resp);
-  ensure_secret_matrix(c, st);
-  if (c.tc_colsum.n < 2 * n_resp) {
-    ck(cudaStreamSynchronize(st), "client sync");
-    c.tc_q.alloc(8ull * n_resp * n);
-    c.tc_colsum.alloc(2 * n_resp);
-    c.tc_ax.alloc(4 * n_resp * n);
-  }
-  uint64_t inv = 0;
-  if (!opir::invert_mod(kSplitP1 % kSplitP2, kSplitP2, inv)) throw std::runtime_error("split primes");
-  ck(cudaMemsetAsync(c.tc_err.p, 0, sizeof(uint32_t), st), "scan error reset");
-  k_client_tc_prep_split<<<nr, kBlock, 0, st>>>(resp, n, nr, c.params.small_q, c.tc_q.p,
-                                                c.tc_colsum.p);
-  launched("client prep launch");
-  const uint64_t plane_set = 4ull * n_resp * n, out = n_resp * n;
-  for (int hf = 0; hf < 2; ++hf)
-    for (int pr = 0; pr < 2; ++pr)
-      scan_secret_matrix(c, nr, pr ? kSplitP2 : kSplitP1, c.tc_q.p + hf * plane_set,
-                         c.tc_ax.p + (2 * hf + pr) * out, st);
-  k_client_tc_finish_split<<<nr, kBlock, 0, st>>>(resp, c.tc_ax.p, c.tc_colsum.p, n, nr, kSplitP1,
-                                                  kSplitP2, inv, dec_const(c.params), pt, noise);
-  launched("client finish launch");
-  check_scan_error(c, st, "client decrypt");
-}
-
+// Plane counts of a reduced response: 3 (narrow moduli, small_q below 2^24), 4
+// (below 2^29) or 7 (below 2^50).
 void launch_decrypt_tc(uint64_t n_resp, cudaStream_t st, const uint64_t *resp, opir_client &c,
                        uint64_t *pt, unsigned long long *noise) {
-  if (c.params.small_q >= (1ull << 29))
-    return launch_decrypt_tc_split(n_resp, st, resp, c, pt, noise);
   const uint32_t n = c.n, nr = static_cast<uint32_t>(n_resp);
-  const uint64_t sq = c.params.small_q;
   ensure_secret_matrix(c, st);
-  if (c.tc_colsum.n < n_resp) {
-    ck(cudaStreamSynchronize(st), "client sync");
-    c.tc_q.alloc(4ull * n_resp * n);
-    c.tc_colsum.alloc(n_resp);
-    c.tc_ax.alloc(n_resp * n);
-  }
-  ck(cudaMemsetAsync(c.tc_err.p, 0, sizeof(uint32_t), st), "scan error reset");
-  k_client_tc_prep<<<nr, kBlock, 0, st>>>(resp, n, nr, sq, c.tc_q.p, c.tc_colsum.p);
-  launched("client prep launch");
-  scan_secret_matrix(c, nr, sq, c.tc_q.p, c.tc_ax.p, st);
-  k_client_tc_finish<<<nr, kBlock, 0, st>>>(resp, c.tc_ax.p, c.tc_colsum.p, n,
-                                            dec_const(c.params), pt, noise);
-  launched("client finish launch");
-  // the scan's bounded waits report through its error word
-  check_scan_error(c, st, "client decrypt");
+  FinishDecrypt fin{};
+  fin.resp = resp;
+  fin.pt = pt;
+  fin.noise = noise;
+  fin.dc = dec_const(c.params);
+  fin.n = n;
+  const uint64_t sq = c.params.small_q;
+  fin.bias = sq * (2ull * n + 1);
+  const auto run = [&](auto np) {
+    constexpr int NP = decltype(np)::value;
+    ensure_planes(c, NP, n_resp, st);
+    if (NP > 4) fin.mod = big_mod(sq, n, 32, 18);  // sq < 2^50
+    k_client_planes<NP><<<nr, kBlock, 0, st>>>(resp + n, 2ull * n, n, nr, sq, fin.dc.mu_sq, c.tc_q.p,
+                                               c.tc_colsum.p, nullptr, 1);
+    launched("client planes launch");
+    secret_product<NP>(c, n_resp, c.tc_q.p, c.tc_colsum.p, fin, st);
+  };
+  if (fin.dc.narrow) run(std::integral_constant<int, 3>{});
+  else if (sq < (1ull << 29)) run(std::integral_constant<int, 4>{});
+  else run(std::integral_constant<int, 7>{});
+  check_product_error(c, st, "client decrypt");
 }
 
 void launch_decrypt(uint64_t n_resp, cudaStream_t st, const uint64_t *resp, const opir_client &c,
@@ -1492,13 +1616,9 @@ void opir_client_destroy(opir_client *c) {
     c->tc_a.reset();
     c->tc_q.reset();
     c->tc_colsum.reset();
-    c->tc_ax.reset();
-    c->tc_err.reset();
-    c->pk_q.reset();
+    if (c->tc_err) error_words().give_back(c->tc_err);
     c->pk_idx.reset();
     if (c->idx_staging) cudaFreeHost(c->idx_staging);
-    c->pk_colsum.reset();
-    c->pk_ax.reset();
     c->consts.reset();
     if (c->staging) cudaFreeHost(c->staging);
     if (c->staged) cudaEventDestroy(c->staged);

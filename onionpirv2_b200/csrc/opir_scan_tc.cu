@@ -60,14 +60,6 @@ constexpr int kEpilogueThreads = 256;
 constexpr size_t kBarrierBytes = 256;  // mbarriers, TMEM slot, abort flag
 constexpr uint32_t kTmemCols = 512;
 
-// x mod q with mu = floor((2^64 - 1) / q), by Barrett's 64-bit quotient.
-__device__ __forceinline__ uint32_t reduce64_barrett(uint64_t x, uint32_t q, uint64_t mu) {
-  const uint64_t qhat = __umul64hi(x, mu);
-  uint64_t r = x - qhat * q;
-  if (r >= q) r -= q;
-  if (r >= q) r -= q;
-  return static_cast<uint32_t>(r);
-}
 // x mod q for any 64-bit x, from one 32-bit high product when mu = floor((2^64
 // - 1) / q) = 8 2^32 + mu_lo (the 29-bit residues; the launcher checks),
 // so with x = xh 2^32 + xl, x mu / 2^64 = 8 xh + xh mu_lo / 2^32 + xl / 2^29
@@ -83,9 +75,7 @@ __device__ __forceinline__ uint32_t reduce64_tc(uint64_t x, uint32_t q, uint64_t
   return min(r, r - q);
 }
 
-// FAST: every residue's mu is 8 2^32 + mu_lo (reduce64_tc), else Barrett
-// (the client's one-residue products mod small_q use the same kernel).
-template <int KT, bool FAST>
+template <int KT>
 __global__ void __launch_bounds__(kThreadsTc, 1)
 k_scan_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmQ,
           TcScanArgs a) {
@@ -272,7 +262,7 @@ k_scan_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
           }
 #pragma unroll
           for (int c = 0; c < 8; ++c)
-            outv[8 * cc + c] = FAST ? reduce64_tc(acc[c], q, mu) : reduce64_barrett(acc[c], q, mu);
+            outv[8 * cc + c] = reduce64_tc(acc[c], q, mu);
         }
         if (last) {  // the accumulators are in registers: hand the TMEM set back first
           fence_before();
@@ -329,10 +319,8 @@ void configure_scan_tc() {
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
   if (done.count(dev)) return;
-  for (const void *k : {reinterpret_cast<const void *>(k_scan_tc<128, true>),
-                        reinterpret_cast<const void *>(k_scan_tc<64, true>),
-                        reinterpret_cast<const void *>(k_scan_tc<128, false>),
-                        reinterpret_cast<const void *>(k_scan_tc<64, false>)}) {
+  for (const void *k : {reinterpret_cast<const void *>(k_scan_tc<128>),
+                        reinterpret_cast<const void *>(k_scan_tc<64>)}) {
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                static_cast<int>(kSmemLimit));
     if (e != cudaSuccess)
@@ -421,15 +409,12 @@ void launch_scan_tc(const CUtensorMap &mapA, const CUtensorMap &mapQ, const TcSc
   const unsigned grid = static_cast<unsigned>(items < static_cast<uint64_t>(sm_count) ? items : sm_count);
   TcScanArgs a = args;  // 0: the default limit (~1 s)
   if (a.wait_cycles <= 0) a.wait_cycles = tc::kWaitCycles;
-  const bool fast = (a.mu[0] >> 32) == 8 && (a.mu[1] >> 32) == 8;
-  if (a.kt == 128 && fast)
-    k_scan_tc<128, true><<<grid, kThreadsTc, smem, st>>>(mapA, mapQ, a);
-  else if (a.kt == 128)
-    k_scan_tc<128, false><<<grid, kThreadsTc, smem, st>>>(mapA, mapQ, a);
-  else if (fast)
-    k_scan_tc<64, true><<<grid, kThreadsTc, smem, st>>>(mapA, mapQ, a);
+  if ((a.mu[0] >> 32) != 8 || (a.mu[1] >> 32) != 8)
+    throw std::invalid_argument("tensor-core scan: moduli with floor(2^64 / q) = 8 2^32 + mu_lo only");
+  if (a.kt == 128)
+    k_scan_tc<128><<<grid, kThreadsTc, smem, st>>>(mapA, mapQ, a);
   else
-    k_scan_tc<64, false><<<grid, kThreadsTc, smem, st>>>(mapA, mapQ, a);
+    k_scan_tc<64><<<grid, kThreadsTc, smem, st>>>(mapA, mapQ, a);
   note_launches(1);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string("k_scan_tc: ") + cudaGetErrorString(e));
