@@ -741,21 +741,22 @@ k_selectors(DevParams P, Shape S, const uint32_t *__restrict__ leaves, uint64_t 
 // Forward NTT of the first n0 leaves (prep_query_composite, server.cpp:
 // 264-304) into `out`, same ciphertext layout as the leaves, stored as
 // coalesced quads; k_fst_pack then turns them into byte planes.
-constexpr int kFstTile = 4;  // ciphertexts per block (8 planes)
+// Tile ciphertexts (2 Tile planes) per block.
+constexpr int kFstTile = 4;
 
-template <int RES>
+template <int RES, int Tile>
 __device__ __forceinline__ void fst_ntt_body(const DevParams &P, const Shape &S,
                                              const uint32_t *leaves, uint64_t leaf_stride,
                                              uint32_t *out, uint64_t out_stride) {
   extern __shared__ uint32_t sm[];
   const int b = blockIdx.z, tid = threadIdx.x;
-  const uint32_t k0 = blockIdx.x * kFstTile;
+  const uint32_t k0 = blockIdx.x * Tile;
   const ResidueTables &T = P.r[RES];
   {
     // every plane's loads first (more loads in flight), then the first pass
-    uint32_t v[2 * kFstTile][8];
+    uint32_t v[2 * Tile][8];
 #pragma unroll
-    for (int e = 0; e < 2 * kFstTile; ++e) {
+    for (int e = 0; e < 2 * Tile; ++e) {
       const uint32_t kk = k0 + (e >> 1);
       const int p = e & 1;
       const uint32_t *src = leaves + ((uint64_t)b * leaf_stride + kk) * kCtWords + (p * 2 + RES) * kN;
@@ -763,17 +764,17 @@ __device__ __forceinline__ void fst_ntt_body(const DevParams &P, const Shape &S,
       for (int k = 0; k < 8; ++k) v[e][k] = kk < S.n0 ? src[posA(tid, k)] : 0u;
     }
 #pragma unroll
-    for (int e = 0; e < 2 * kFstTile; ++e) {
+    for (int e = 0; e < 2 * Tile; ++e) {
       fA<RES>(v[e]);
       st_plane<0>(sm + e * kPad, v[e], tid);
     }
   }
   __syncthreads();
-  fwd_mid_r<RES>(sm, 2 * kFstTile, T.fwt);
+  fwd_mid_r<RES>(sm, 2 * Tile, T.fwt);
   uint2 wd[6];
   fload_d(wd, T.fwt, tid);
 #pragma unroll
-  for (int e = 0; e < 2 * kFstTile; ++e) {
+  for (int e = 0; e < 2 * Tile; ++e) {
     const uint32_t kk = k0 + (e >> 1);
     if (kk >= S.n0) continue;  // uniform over the block
     const int p = e & 1;
@@ -790,13 +791,14 @@ __device__ __forceinline__ void fst_ntt_body(const DevParams &P, const Shape &S,
   }
 }
 
+template <int Tile>
 __global__ void __launch_bounds__(kThreads, 2)
 k_fst_ntt(DevParams P, Shape S, const uint32_t *__restrict__ leaves, uint64_t leaf_stride,
           uint32_t *__restrict__ out, uint64_t out_stride) {
   if (blockIdx.y == 0)
-    fst_ntt_body<0>(P, S, leaves, leaf_stride, out, out_stride);
+    fst_ntt_body<0, Tile>(P, S, leaves, leaf_stride, out, out_stride);
   else
-    fst_ntt_body<1>(P, S, leaves, leaf_stride, out, out_stride);
+    fst_ntt_body<1, Tile>(P, S, leaves, leaf_stride, out, out_stride);
 }
 
 // Byte-plane packing of the NTT-form query matrix:
@@ -992,6 +994,85 @@ k_scan_epilogue(DevParams P, Shape S, const uint32_t *__restrict__ cmat, uint32_
     scan_epilogue_body<0, VEC>(P, S, cmat, ncols, mid, mid_stride);
   else
     scan_epilogue_body<1, VEC>(P, S, cmat, ncols, mid, mid_stride);
+}
+
+// ------------------------------------------- first dimension row by row
+// One database row (rows[blockIdx.x], any handle's) times the n0 NTT-form
+// ciphertexts of one query, then the inverse NTT: one residue and polynomial
+// per CTA. For first dimensions so short that the tensor-core scan is padding
+// (a 128 x 128-byte tile per level for 8 columns took 43 us a database; a
+// tree has one database per level): every thread reads its eight levels' 16
+// bytes per plane, sums exact 64-bit products (n0 <= 64 of 29 x 29 bits) and
+// keeps them for the inverse transform. 21 rows of 17 databases: one launch
+// of 16 us. Bound by its chain of loads and the transform's latency.
+template <int RES>
+__device__ __forceinline__ void rows_first_dim_body(const DevParams &P, const FirstDimRow &row,
+                                                    uint32_t n0, uint32_t n0p, const uint32_t *ntt) {
+  extern __shared__ uint32_t sm[];
+  const int tid = threadIdx.x, p = blockIdx.z;
+  const ResidueTables &T = P.r[RES];
+  const uint32_t *q = ntt + (p * 2 + RES) * kN;
+  uint64_t acc[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) acc[k] = 0;
+  for (uint32_t k0 = 0; k0 < n0p; k0 += 16) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int j0 = 4 * (tid + 256 * h);
+      uint32_t a[4][16];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const uint8_t *d = row.db + (static_cast<uint64_t>(RES) * kN + j0 + c) * 4 * row.plane + k0;
+        unpack16(__ldg(reinterpret_cast<const uint4 *>(d)),
+                 __ldg(reinterpret_cast<const uint4 *>(d + row.plane)),
+                 __ldg(reinterpret_cast<const uint4 *>(d + 2 * row.plane)),
+                 __ldg(reinterpret_cast<const uint4 *>(d + 3 * row.plane)), a[c]);
+      }
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        if (k0 + k >= n0) break;  // uniform over the block
+        const uint4 x = __ldg(reinterpret_cast<const uint4 *>(q + static_cast<uint64_t>(k0 + k) * kCtWords + j0));
+        acc[4 * h + 0] += static_cast<uint64_t>(a[0][k]) * x.x;
+        acc[4 * h + 1] += static_cast<uint64_t>(a[1][k]) * x.y;
+        acc[4 * h + 2] += static_cast<uint64_t>(a[2][k]) * x.z;
+        acc[4 * h + 3] += static_cast<uint64_t>(a[3][k]) * x.w;
+      }
+    }
+  }
+  uint32_t v[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = red64_lazy<RES>(acc[k]);
+  {
+    uint2 wd[6];
+    iload_d(wd, T.iwt, tid);
+    iD<RES>(v, wd);
+  }
+  st_plane<3>(sm, v, tid);
+  __syncthreads();
+  inv_mid_r<RES, false>(sm, 1, T.iwt);
+  ld_plane<0>(sm, v, tid);
+  iA<RES>(v);
+  uint32_t *o = row.out + (p * 2 + RES) * kN;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) o[posA(tid, k)] = v[k];
+}
+__global__ void __launch_bounds__(kThreads)
+k_rows_first_dim(DevParams P, const FirstDimRow *__restrict__ rows, uint32_t n0, uint32_t n0p,
+                 const uint32_t *__restrict__ ntt) {
+  const FirstDimRow row = rows[blockIdx.x];
+  if (blockIdx.y == 0)
+    rows_first_dim_body<0>(P, row, n0, n0p, ntt);
+  else
+    rows_first_dim_body<1>(P, row, n0, n0p, ntt);
+}
+
+// Residue pairs of the ciphertext at cts[blockIdx.y] -> boundary form (one
+// logical modulus), item blockIdx.y of out.
+__global__ void __launch_bounds__(kThreads)
+k_compose_rows(DevParams P, const uint32_t *const *__restrict__ cts, uint64_t *__restrict__ out) {
+  const uint32_t i = blockIdx.x * kThreads + threadIdx.x, p = i >> kLogN, j = i & (kN - 1);
+  const uint32_t *s = cts[blockIdx.y] + p * 2 * kN + j;
+  out[static_cast<uint64_t>(blockIdx.y) * 2 * kN + i] = crt_compose(s[0], s[kN], P);
 }
 
 // --------------------------------------------------------------- MUX level
@@ -1575,15 +1656,47 @@ void launch_selectors(const DevParams &P, const Shape &s, const uint32_t *leaves
     selectors_impl<GadgetsK1Comp>(P, s, leaves, leaf_stride, gsw_keys, sel, batch, st);
 }
 
+void launch_fst_ntt(const DevParams &P, const Shape &s, const uint32_t *leaves,
+                    uint64_t leaf_stride, uint32_t *ntt, uint64_t ntt_stride, uint32_t batch,
+                    cudaStream_t st) {
+  // four leaves per block share their twiddles; one per block when that
+  // leaves SMs idle (8 leaves, one query: 22 us with four, 6 us with one)
+  const uint32_t tiles = (s.n0 + kFstTile - 1) / kFstTile;
+  if (2ull * tiles * batch < static_cast<uint64_t>(sm_count())) {
+    const size_t smem = 2 * kPad * sizeof(uint32_t);
+    set_smem(k_fst_ntt<1>, smem);
+    k_fst_ntt<1><<<dim3(s.n0, 2, batch), kThreads, smem, st>>>(P, s, leaves, leaf_stride, ntt, ntt_stride);
+  } else {
+    const size_t smem = 2 * kFstTile * kPad * sizeof(uint32_t);
+    set_smem(k_fst_ntt<kFstTile>, smem);
+    k_fst_ntt<kFstTile><<<dim3(tiles, 2, batch), kThreads, smem, st>>>(P, s, leaves, leaf_stride, ntt,
+                                                                       ntt_stride);
+  }
+  check_launch("k_fst_ntt");
+}
+
 void launch_fst_prep(const DevParams &P, const Shape &s, const uint32_t *leaves,
                      uint64_t leaf_stride, uint32_t *ntt, uint64_t ntt_stride, uint8_t *qb,
                      uint32_t batch, cudaStream_t st) {
-  const size_t smem = 2 * kFstTile * kPad * sizeof(uint32_t);
-  set_smem(k_fst_ntt, smem);
-  dim3 grid((s.n0 + kFstTile - 1) / kFstTile, 2, batch);
-  k_fst_ntt<<<grid, kThreads, smem, st>>>(P, s, leaves, leaf_stride, ntt, ntt_stride);
-  check_launch("k_fst_ntt");
+  launch_fst_ntt(P, s, leaves, leaf_stride, ntt, ntt_stride, batch, st);
   launch_fst_pack(s, ntt, ntt_stride, qb, batch, st);
+}
+
+void launch_rows_first_dim(const DevParams &P, const FirstDimRow *rows, uint32_t n_rows,
+                           uint32_t n0, uint32_t n0p, const uint32_t *ntt, cudaStream_t st) {
+  if (n_rows == 0) return;
+  if (n0p > kMaxRowsN0 || n0p % 16 != 0 || n0 > n0p)
+    throw std::invalid_argument("row-wise first dimension: first dimension out of range");
+  const size_t smem = kPad * sizeof(uint32_t);
+  k_rows_first_dim<<<dim3(n_rows, 2, 2), kThreads, smem, st>>>(P, rows, n0, n0p, ntt);
+  check_launch("k_rows_first_dim");
+}
+
+void launch_compose_rows(const DevParams &P, const uint32_t *const *cts, uint32_t n, uint64_t *out,
+                         cudaStream_t st) {
+  if (n == 0) return;
+  k_compose_rows<<<dim3(2 * kN / kThreads, n), kThreads, 0, st>>>(P, cts, out);
+  check_launch("k_compose_rows");
 }
 
 void launch_fst_pack(const Shape &s, const uint32_t *ntt, uint64_t ntt_stride, uint8_t *qb,

@@ -93,6 +93,11 @@ void upload_ntt_constants(const uint32_t q[2], const uint32_t *const fw[2],
 void launch_fst_prep(const DevParams &P, const Shape &s, const uint32_t *leaves,
                      uint64_t leaf_stride, uint32_t *ntt, uint64_t ntt_stride, uint8_t *qb,
                      uint32_t batch, cudaStream_t st);
+// The forward NTT alone: the first n0 leaves of each query into `ntt`, the
+// ciphertext layout of the leaves.
+void launch_fst_ntt(const DevParams &P, const Shape &s, const uint32_t *leaves,
+                    uint64_t leaf_stride, uint32_t *ntt, uint64_t ntt_stride, uint32_t batch,
+                    cudaStream_t st);
 // The byte-plane transpose alone, for leaves already in NTT form (the last
 // expansion level's NTT-form children).
 void launch_fst_pack(const Shape &s, const uint32_t *ntt, uint64_t ntt_stride, uint8_t *qb,
@@ -105,6 +110,24 @@ void launch_fst_pack(const Shape &s, const uint32_t *ntt, uint64_t ntt_stride, u
 void launch_scan(const DevParams &P, const Shape &s, const uint8_t *db8,
                  const uint8_t *qb, uint32_t *cmat, uint32_t batch,
                  cudaStream_t st);
+
+// A database row of n0p byte-plane columns (level z, byte plane j at
+// db + (4 z + j) plane) and the ciphertext its product goes to.
+struct FirstDimRow {
+  const uint8_t *db;
+  uint64_t plane;  // bytes between byte planes: rows of the database x n0p
+  uint32_t *out;
+};
+// First dimension of one query over single rows (device array, rows of one or
+// several databases of the same n0): the row times the n0 NTT-form
+// ciphertexts `ntt` (launch_fst_ntt), in coefficient form. n0p <= kMaxRowsN0.
+constexpr uint32_t kMaxRowsN0 = 64;
+void launch_rows_first_dim(const DevParams &P, const FirstDimRow *rows, uint32_t n_rows,
+                           uint32_t n0, uint32_t n0p, const uint32_t *ntt, cudaStream_t st);
+// Residue-pair ciphertexts at n device pointers (device array) -> n x 2N u64
+// mod q1 q2.
+void launch_compose_rows(const DevParams &P, const uint32_t *const *cts, uint32_t n, uint64_t *out,
+                         cudaStream_t st);
 
 // Gather + INTT of the scan output into candidate ciphertexts
 // (src/server.cpp:529-597). mid: batch x mid_stride cts (coefficient form).

@@ -155,8 +155,12 @@ struct opir_tree {
   std::vector<opir_server *> levels;
   cudaStream_t stream = nullptr;
   DevBuf<uint64_t> out;            // (L + 1) x 2N u64
-  cudaEvent_t q_done = nullptr;
+  cudaEvent_t q_done = nullptr, first_done = nullptr;
   std::vector<cudaEvent_t> done;   // per level
+  // short first dimensions (n0 <= kMaxRowsN0): every level's rows, answered in
+  // one launch, and every level's selected ciphertext
+  DevBuf<opir::FirstDimRow> rows;
+  DevBuf<const uint32_t *> selected;
   std::string last_error;
 };
 
@@ -914,6 +918,61 @@ void combine_k1(opir_server *s, uint32_t n, const uint64_t *d_partials, uint64_t
                            n, s->stream);
   opir::launch_modswitch(s->dp, s->comb[cur].p, G, d_resp, nullptr, resp_bytes_of(s->params), n,
                          s->stream);
+}
+
+// opir_tree_query over short first dimensions, from the query's ciphertext in
+// slot 0 of the query handle. The selected ciphertexts depend on the alpha
+// ciphertexts and the beta selectors alone (the gamma bits choose a
+// coefficient, which the client does), so only their leaves are expanded and
+// only the beta selectors completed. The alphas are transformed once for all
+// levels, and one launch takes every level's rows through its first dimension
+// while the selectors are completed on the other stream.
+void tree_query_rows(opir_tree *t, uint64_t *selected) {
+  opir_server *q = t->q;
+  opir::Shape sh = q->shape;
+  const uint64_t slots = q->lvl_slots;
+  sh.num_dims = 1 + static_cast<uint32_t>(t->tree.b);
+  sh.useful = sh.n0 + sh.l_ep * static_cast<uint32_t>(t->tree.b);
+  const uint64_t bv_level_stride = static_cast<uint64_t>(sh.l_ks) * 4 * kN;
+  for (uint32_t d = 0; d < sh.h; ++d)
+    opir::launch_expand_level(q->dp, sh, d, q->lvl[d & 1].p, slots, q->lvl[(d + 1) & 1].p, slots,
+                              q->keyptrs.p, bv_level_stride, 1, q->stream);
+  const uint32_t *leaves = q->lvl[sh.h & 1].p;
+  uint32_t *ntt = q->lvl[(sh.h + 1) & 1].p;
+  ck(cudaEventRecord(t->q_done, q->stream), "event record");
+  ck(cudaStreamWaitEvent(t->stream, t->q_done, 0), "wait");
+  opir::launch_fst_ntt(q->dp, sh, leaves, slots, ntt, slots, 1, t->stream);
+  opir::launch_rows_first_dim(q->dp, t->rows.p, static_cast<uint32_t>(t->rows.n), sh.n0,
+                              t->levels[0]->shape.n0p, ntt, t->stream);
+  ck(cudaEventRecord(t->first_done, t->stream), "event record");
+  opir::launch_selectors(q->dp, sh, leaves, slots, q->keyptrs.p + 1, q->sel.p, 1, q->stream);
+  ck(cudaEventRecord(t->q_done, q->stream), "event record");
+  const uint64_t sel_words = 2ull * sh.l_ep * kCtWords;  // u32 words per selector
+  for (size_t l = 0; l < t->levels.size(); ++l) {
+    opir_server *ls = t->levels[l];
+    const uint32_t fold = static_cast<uint32_t>(ls->fold_count);
+    if (fold == 0) continue;
+    ck(cudaStreamWaitEvent(ls->stream, t->first_done, 0), "wait");
+    ck(cudaStreamWaitEvent(ls->stream, t->q_done, 0), "wait");
+    for (uint32_t a = 1; a <= fold; ++a) {  // MSB-first: step a takes beta bit begin+count-a
+      const uint64_t u = ls->fold_begin + ls->fold_count - a;
+      // step a reads selector slot a: the base for which that is selector u
+      const uint32_t *slot0 = reinterpret_cast<const uint32_t *>(
+          reinterpret_cast<uintptr_t>(q->sel.p + u * sel_words) - a * sel_words * 4);
+      opir::launch_mux_level(ls->dp, ls->shape, a, ls->shape.num_dims - 1, ls->mid[(a - 1) & 1].p,
+                             ls->mid[a & 1].p, ls->shape.other, slot0, 1, ls->stream);
+    }
+    ck(cudaEventRecord(t->done[l], ls->stream), "event record");
+    ck(cudaStreamWaitEvent(t->stream, t->done[l], 0), "wait");
+  }
+  // the query handle's selectors finish before its buffers are used again,
+  // also when no level folds
+  ck(cudaStreamWaitEvent(t->stream, t->q_done, 0), "wait");
+  opir::launch_compose_rows(q->dp, t->selected.p, static_cast<uint32_t>(t->levels.size()), t->out.p,
+                            t->stream);
+  ck(cudaMemcpyAsync(selected, t->out.p, t->levels.size() * 2ull * kN * 8, cudaMemcpyDeviceToHost,
+                     t->stream), "download");
+  ck(cudaStreamSynchronize(t->stream), "tree query");
 }
 
 // Orders the handle's stream after the caller's work on `user` (if any).
@@ -1982,7 +2041,10 @@ void opir_tree_destroy(opir_tree *t) {
     if (t->q) opir_server_destroy(t->q);
     for (cudaEvent_t e : t->done) cudaEventDestroy(e);
     if (t->q_done) cudaEventDestroy(t->q_done);
+    if (t->first_done) cudaEventDestroy(t->first_done);
     t->out.reset();
+    t->rows.reset();
+    t->selected.reset();
     if (t->stream) cudaStreamDestroy(t->stream);
     if (prev >= 0) cudaSetDevice(prev);
   }
@@ -2020,6 +2082,7 @@ opir_status opir_tree_create(const opir_params *scheme, const opir_tree_params *
     DeviceGuard g(device);
     ck(cudaStreamCreateWithFlags(&t->stream, cudaStreamNonBlocking), "cudaStreamCreate");
     ck(cudaEventCreateWithFlags(&t->q_done, cudaEventDisableTiming), "event");
+    ck(cudaEventCreateWithFlags(&t->first_done, cudaEventDisableTiming), "event");
     t->done.resize(t->levels.size(), nullptr);
     for (auto &e : t->done) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
     // no allocation while answering
@@ -2032,6 +2095,24 @@ opir_status opir_tree_create(const opir_params *scheme, const opir_tree_params *
       ensure_capacity(t->q, 1);
       grow_keyptr_slots(t->q, 2);
       for (opir_server *l : t->levels) ensure_capacity(l, 1);
+      if (t->q->shape.n0 <= opir::kMaxRowsN0) {
+        std::vector<opir::FirstDimRow> rows;
+        std::vector<const uint32_t *> selected;
+        for (opir_server *l : t->levels) {
+          const opir::Shape &sh = l->shape;
+          for (uint32_t r = 0; r < sh.other; ++r)
+            rows.push_back({l->db8.p + static_cast<uint64_t>(r) * sh.n0p,
+                            static_cast<uint64_t>(sh.other) * sh.n0p,
+                            l->mid[0].p + static_cast<uint64_t>(r) * kCtWords});
+          selected.push_back(l->mid[l->fold_count & 1].p);
+        }
+        t->rows.alloc(rows.size());
+        t->selected.alloc(selected.size());
+        ck(cudaMemcpy(t->rows.p, rows.data(), rows.size() * sizeof(rows[0]), cudaMemcpyHostToDevice),
+           "tree rows");
+        ck(cudaMemcpy(t->selected.p, selected.data(), selected.size() * sizeof(selected[0]),
+                      cudaMemcpyHostToDevice), "tree rows");
+      }
     }
   });
   if (st != OPIR_OK) {
@@ -2082,6 +2163,10 @@ opir_status opir_tree_query(opir_tree *t, uint64_t client_id, const uint64_t *qu
     upload_keyptrs(q, &client_id, 1);
     ck(cudaMemcpyAsync(q->q_u64.p, query, 2 * kN * 8, cudaMemcpyHostToDevice, q->stream), "upload");
     opir::launch_split_u64(q->dp, q->q_u64.p, q->lvl[0].p, 1, 2, q->lvl_slots * kCtWords, q->stream);
+    if (t->rows.n) {
+      tree_query_rows(t, selected);
+      return;
+    }
     const uint32_t *leaves = run_expand(q, 1);
     opir::launch_selectors(q->dp, q->shape, leaves, q->lvl_slots, q->keyptrs.p + 1, q->sel.p, 1,
                            q->stream);
