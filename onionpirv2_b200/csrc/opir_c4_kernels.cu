@@ -1148,14 +1148,14 @@ k4_modswitch(Dev4 P, const uint64_t *__restrict__ ct_all, uint64_t ct_stride,
   extern __shared__ uint64_t vals[];  // 2N
   const int b = blockIdx.x;
   const uint64_t *ct = ct_all + static_cast<uint64_t>(b) * ct_stride * kCtWords;
-  for (int idx = threadIdx.x; idx < 2 * kN; idx += blockDim.x) {
+  for (int idx = blockIdx.y * blockDim.x + threadIdx.x; idx < 2 * kN; idx += gridDim.y * blockDim.x) {
     const int p = idx >> 12, j = idx & (kN - 1);
     const u128 x = compose(ct[p * 2 * kN + j], ct[p * 2 * kN + kN + j], P.q0inv, P.q0inv_sh);
     uint64_t v = static_cast<uint64_t>((x + (static_cast<u128>(kQ1) >> 1)) / kQ1);
     if (v >= kQ0) v -= kQ0;
     const uint64_t r = rescale_dev(v, kQ0, P.small_q);
     resp[static_cast<uint64_t>(b) * 2 * kN + idx] = r;
-    vals[idx] = r & ((1ull << P.small_q_width) - 1);
+    if (bytes) vals[idx] = r & ((1ull << P.small_q_width) - 1);
   }
   if (bytes == nullptr) return;
   __syncthreads();
@@ -1386,9 +1386,13 @@ void launch_mux_level(const Dev4 &P, const Shape4 &s, uint32_t level, uint32_t t
 
 void launch_modswitch(const Dev4 &P, const uint64_t *ct, uint64_t ct_stride, uint64_t *resp,
                       uint8_t *bytes, uint32_t resp_bytes, uint32_t batch, cudaStream_t st) {
-  const size_t smem = 2 * kN * sizeof(uint64_t);
-  set_smem(k4_modswitch, smem);
-  k4_modswitch<<<batch, 256, smem, st>>>(P, ct, ct_stride, resp, bytes, resp_bytes);
+  // one coefficient per thread: its two 128-bit divisions are a serial chain
+  // (one block per query took 73 us of a lone query); packing needs every
+  // value in one block
+  const size_t smem = bytes ? 2 * kN * sizeof(uint64_t) : 0;
+  if (smem) set_smem(k4_modswitch, smem);
+  k4_modswitch<<<dim3(batch, bytes ? 1 : 2 * kN / 256), 256, smem, st>>>(P, ct, ct_stride, resp, bytes,
+                                                                        resp_bytes);
   check_launch("k4_modswitch");
 }
 

@@ -925,7 +925,7 @@ k1p_modswitch(Dev1 P, const uint64_t *__restrict__ ct_all, uint64_t ct_stride,
   extern __shared__ uint64_t vals[];  // 2N when packing
   const int b = blockIdx.x;
   const uint64_t *ct = ct_all + static_cast<uint64_t>(b) * ct_stride * kCtWords;
-  for (int idx = threadIdx.x; idx < 2 * kN; idx += blockDim.x) {
+  for (int idx = blockIdx.y * blockDim.x + threadIdx.x; idx < 2 * kN; idx += gridDim.y * blockDim.x) {
     const uint64_t r = rescale_q(ct[idx], P.small_q);
     resp[static_cast<uint64_t>(b) * 2 * kN + idx] = r;
     if (bytes) vals[idx] = r;
@@ -1109,7 +1109,10 @@ void launch_modswitch(const Dev1 &P, const uint64_t *ct, uint64_t ct_stride, uin
                       uint8_t *bytes, uint32_t resp_bytes, uint32_t batch, cudaStream_t st) {
   const size_t smem = bytes ? 2 * kN * sizeof(uint64_t) : 0;
   if (smem) set_smem(k1p_modswitch, smem);
-  k1p_modswitch<<<batch, 256, smem, st>>>(P, ct, ct_stride, resp, bytes, resp_bytes);
+  // one coefficient per thread (a 128-bit division each); packing needs
+  // every value in one block
+  k1p_modswitch<<<dim3(batch, bytes ? 1 : 2 * kN / 256), 256, smem, st>>>(P, ct, ct_stride, resp, bytes,
+                                                                         resp_bytes);
   check_launch("k1p_modswitch");
 }
 
