@@ -14,14 +14,15 @@
 // w[2b + 2g (+1)] (stage 2), w[4b + 4g + 0..3] (stage 3): A (1, 0),
 // B (8, t >> 6), C (64, t >> 3), D (512, t). Merged Cooley-Tukey forward with
 // bit-reversed output and Gentleman-Sande inverse scaled by N^-1, the HEXL
-// convention of the reference (utils.cpp:26-56). Forward butterflies are
-// Harvey/Shoup lazy with X corrected only on stages 4, 6, 8, 10, 12 (values
-// stay below 8q < 2^63, outputs below 6q); inverse ones keep [0, 2q).
+// convention of the reference (utils.cpp:26-56). Butterflies fold modulo
+// q = 2^60 - c (opir_fold60.cuh): forward values grow by about q a stage from
+// [q, 2q) and stay below 2^64, inverse passes begin and end folded.
 #pragma once
 
 #include <cstdint>
 
 #include "opir_c4_kernels.h"
+#include "opir_fold60.cuh"
 
 namespace opir4 {
 
@@ -33,10 +34,10 @@ struct Limb {
   static constexpr uint64_t q = L ? kQ1 : kQ0;
 };
 
-// (w, floor(w 2^64 / q)) for twiddle indices < 64: [limb][index]
+// opir60::twiddle() of the twiddles with index < 64: [limb][index]
 static __constant__ ulonglong2 c4_fwt[2][64];
 static __constant__ ulonglong2 c4_iwt[2][64];
-// {N^-1, Shoup} and {iw[1] N^-1, Shoup} per limb
+// N^-1 and iw[1] N^-1 per limb
 static __constant__ ulonglong2 c4_ninv[2], c4_w1ninv[2];
 
 __device__ __forceinline__ int pad(int p) { return p + (p >> 3); }
@@ -45,16 +46,11 @@ __device__ __forceinline__ int posB(int t, int k) { return ((t >> 6) << 9) + (t 
 __device__ __forceinline__ int posC(int t, int k) { return ((t >> 3) << 6) + (t & 7) + 8 * k; }
 __device__ __forceinline__ int posD(int t, int k) { return 8 * t + k; }
 
-// a w mod q in [0, 2q) for any 64-bit a (Shoup; ws = floor(w 2^64 / q))
+// a w mod q in [0, 2q) for any 64-bit a (Shoup; ws = floor(w 2^64 / q)): the
+// key rows, which carry that companion
 template <uint64_t Q>
 __device__ __forceinline__ uint64_t mul_shoup(uint64_t a, uint64_t w, uint64_t ws) {
   return a * w - __umul64hi(a, ws) * Q;
-}
-template <uint64_t Q>
-__device__ __forceinline__ uint64_t canon8(uint64_t x) {  // [0, 8q) -> [0, q)
-  x = min(x, x - 4 * Q);
-  x = min(x, x - 2 * Q);
-  return min(x, x - Q);
 }
 template <uint64_t Q>
 __device__ __forceinline__ uint64_t add_mod(uint64_t a, uint64_t b) {
@@ -88,41 +84,6 @@ __device__ __forceinline__ uint64_t red128(unsigned __int128 x) {
 }
 
 // ----------------------------------------------------------------- NTT
-template <uint64_t Q, bool C>
-__device__ __forceinline__ void fbf(uint64_t &X, uint64_t &Y, ulonglong2 w) {
-  uint64_t x = X;
-  if (C) x = min(x, x - 4 * Q);
-  const uint64_t t = mul_shoup<Q>(Y, w.x, w.y);
-  X = x + t;
-  Y = x - t + 2 * Q;
-}
-template <uint64_t Q, bool C1, bool C2, bool C3>
-__device__ __forceinline__ void fpass(uint64_t (&v)[8], const ulonglong2 (&w)[7]) {
-  fbf<Q, C1>(v[0], v[4], w[0]); fbf<Q, C1>(v[1], v[5], w[0]);
-  fbf<Q, C1>(v[2], v[6], w[0]); fbf<Q, C1>(v[3], v[7], w[0]);
-  fbf<Q, C2>(v[0], v[2], w[1]); fbf<Q, C2>(v[1], v[3], w[1]);
-  fbf<Q, C2>(v[4], v[6], w[2]); fbf<Q, C2>(v[5], v[7], w[2]);
-  fbf<Q, C3>(v[0], v[1], w[3]); fbf<Q, C3>(v[2], v[3], w[4]);
-  fbf<Q, C3>(v[4], v[5], w[5]); fbf<Q, C3>(v[6], v[7], w[6]);
-}
-template <uint64_t Q>
-__device__ __forceinline__ void ibf(uint64_t &X, uint64_t &Y, ulonglong2 w) {
-  uint64_t u = X + Y;
-  u = min(u, u - 2 * Q);
-  const uint64_t d = X - Y + 2 * Q;
-  Y = mul_shoup<Q>(d, w.x, w.y);
-  X = u;
-}
-template <uint64_t Q>
-__device__ __forceinline__ void ipass(uint64_t (&v)[8], const ulonglong2 (&w)[7]) {
-  ibf<Q>(v[0], v[1], w[3]); ibf<Q>(v[2], v[3], w[4]);
-  ibf<Q>(v[4], v[5], w[5]); ibf<Q>(v[6], v[7], w[6]);
-  ibf<Q>(v[0], v[2], w[1]); ibf<Q>(v[1], v[3], w[1]);
-  ibf<Q>(v[4], v[6], w[2]); ibf<Q>(v[5], v[7], w[2]);
-  ibf<Q>(v[0], v[4], w[0]); ibf<Q>(v[1], v[5], w[0]);
-  ibf<Q>(v[2], v[6], w[0]); ibf<Q>(v[3], v[7], w[0]);
-}
-
 // twiddles of a pass: base b, group g; constant memory when every index < 64
 template <int L, bool FWD>
 __device__ __forceinline__ void tw_const(ulonglong2 (&w)[7], int b, int g) {
@@ -161,7 +122,7 @@ template <int L>
 __device__ __forceinline__ void fA(uint64_t (&v)[8]) {
   ulonglong2 w[7];
   tw_const<L, true>(w, 1, 0);
-  fpass<Limb<L>::q, false, false, false>(v, w);
+  opir60::fpass8<Limb<L>::q, true>(v, w);
 }
 // Forward passes B and C over np planes stored in A-order (after fA), up to
 // a __syncthreads; ends synchronised. Then: ld_plane<3> + fD.
@@ -176,7 +137,7 @@ __device__ __forceinline__ void fwd_mid(uint64_t *sm, int np, const Tables &T) {
     for (int i = 0; i < np; ++i) {
       uint64_t v[8];
       ld_plane<1>(sm + i * kPad, v, t);
-      fpass<Q, true, false, true>(v, w);
+      opir60::fpass8<Q, false>(v, w);
       st_plane<1>(sm + i * kPad, v, t);
     }
   }
@@ -188,30 +149,30 @@ __device__ __forceinline__ void fwd_mid(uint64_t *sm, int np, const Tables &T) {
     for (int i = 0; i < np; ++i) {
       uint64_t v[8];
       ld_plane<2>(sm + i * kPad, v, t);
-      fpass<Q, false, true, false>(v, w);
+      opir60::fpass8<Q, false>(v, w);
       st_plane<2>(sm + i * kPad, v, t);
     }
   }
   __syncthreads();
 }
-// forward pass D (stages 10-12, D-order values), output in [0, 6q)
+// forward pass D (stages 10-12, D-order values), output any 64 bits
 template <int L>
 __device__ __forceinline__ void fD(uint64_t (&v)[8], const ulonglong2 (&w)[7]) {
-  fpass<Limb<L>::q, true, false, true>(v, w);
+  opir60::fpass8<Limb<L>::q, false>(v, w);
 }
 template <int L>
 __device__ __forceinline__ void fload_d(ulonglong2 (&w)[7], const Tables &T) {
   tw_global(w, T.fwt[L], 512, threadIdx.x);
 }
 
-// inverse: pass D first (D-order, inputs in [0, 2q))
+// inverse: pass D first (D-order, inputs folded)
 template <int L>
 __device__ __forceinline__ void iload_d(ulonglong2 (&w)[7], const Tables &T) {
   tw_global(w, T.iwt[L], 512, threadIdx.x);
 }
 template <int L>
 __device__ __forceinline__ void iD(uint64_t (&v)[8], const ulonglong2 (&w)[7]) {
-  ipass<Limb<L>::q>(v, w);
+  opir60::ipass8<Limb<L>::q>(v, w);
 }
 // Inverse passes C and B over np planes stored in D-order after iD, up to a
 // __syncthreads; ends synchronised. Then: ld_plane<0> + iA.
@@ -226,7 +187,7 @@ __device__ __forceinline__ void inv_mid(uint64_t *sm, int np, const Tables &T) {
     for (int i = 0; i < np; ++i) {
       uint64_t v[8];
       ld_plane<2>(sm + i * kPad, v, t);
-      ipass<Q>(v, w);
+      opir60::ipass8<Q>(v, w);
       st_plane<2>(sm + i * kPad, v, t);
     }
   }
@@ -238,7 +199,7 @@ __device__ __forceinline__ void inv_mid(uint64_t *sm, int np, const Tables &T) {
     for (int i = 0; i < np; ++i) {
       uint64_t v[8];
       ld_plane<1>(sm + i * kPad, v, t);
-      ipass<Q>(v, w);
+      opir60::ipass8<Q>(v, w);
       st_plane<1>(sm + i * kPad, v, t);
     }
   }
@@ -248,20 +209,7 @@ __device__ __forceinline__ void inv_mid(uint64_t *sm, int np, const Tables &T) {
 // distance-2048 stage with N^-1 folded in; output canonical
 template <int L>
 __device__ __forceinline__ void iA(uint64_t (&v)[8]) {
-  constexpr uint64_t Q = Limb<L>::q;
-  ibf<Q>(v[0], v[1], c4_iwt[L][4]); ibf<Q>(v[2], v[3], c4_iwt[L][5]);
-  ibf<Q>(v[4], v[5], c4_iwt[L][6]); ibf<Q>(v[6], v[7], c4_iwt[L][7]);
-  ibf<Q>(v[0], v[2], c4_iwt[L][2]); ibf<Q>(v[1], v[3], c4_iwt[L][2]);
-  ibf<Q>(v[4], v[6], c4_iwt[L][3]); ibf<Q>(v[5], v[7], c4_iwt[L][3]);
-  const ulonglong2 a = c4_ninv[L], b = c4_w1ninv[L];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint64_t X = v[k], Y = v[k + 4];
-    const uint64_t ra = mul_shoup<Q>(X + Y, a.x, a.y);
-    const uint64_t rb = mul_shoup<Q>(X - Y + 2 * Q, b.x, b.y);
-    v[k] = min(ra, ra - Q);
-    v[k + 4] = min(rb, rb - Q);
-  }
+  opir60::ilast8<Limb<L>::q>(v, c4_iwt[L], c4_ninv[L], c4_w1ninv[L]);
 }
 
 // floor(w 2^64 / q) for w < q = 2^60 - c: w 2^64 = w (16 q + 16 c), so the
@@ -277,14 +225,6 @@ __device__ __forceinline__ uint64_t shoup_of(uint64_t w) {
   const uint64_t r0 = (lo & ((1ull << 60) - 1)) + t0 * c;
   return 16 * w + t0 + (r0 >= Q ? 1 : 0);
 }
-// [0, 16q) -> [0, 2q)
-template <uint64_t Q>
-__device__ __forceinline__ uint64_t fold16(uint64_t x) {
-  x = min(x, x - 8 * Q);
-  x = min(x, x - 4 * Q);
-  return min(x, x - 2 * Q);
-}
-
 // ------------------------------------------------------ RNS <-> integer
 // Garner compose of canonical limbs into [0, q0 q1) (gsw.cpp:22-53)
 __device__ __forceinline__ unsigned __int128 compose(uint64_t r0, uint64_t r1, uint64_t q0inv,

@@ -185,7 +185,7 @@ __device__ __forceinline__ void db_body(const Dev4 &P, const uint64_t *coeffs,
     ld_plane<3>(sm4 + e * kPad, out[e], tid);
     fD<L>(out[e], wd);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) out[e][k] = canon8<Limb<L>::q>(out[e][k]);
+    for (int k = 0; k < 8; ++k) out[e][k] = opir60::canon<Limb<L>::q>(out[e][k]);
   }
   const uint64_t row = pt0 / n0, col = pt0 % n0;
   const uint64_t plane_bytes = static_cast<uint64_t>(other) * n0p;
@@ -278,8 +278,8 @@ __device__ __forceinline__ void expand_tail_ntt(const Dev4 &P, uint32_t galois, 
   }
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    h0[k] = canon8<Q>(h0[k]);
-    h1[k] = canon8<Q>(h1[k]);
+    h0[k] = opir60::canon<Q>(h0[k]);
+    h1[k] = opir60::canon<Q>(h1[k]);
   }
   st_plane<3>(sm4 + 2 * kPad, h0, tid);  // c0^ by slot, for the sigma gather
   __syncthreads();
@@ -294,8 +294,8 @@ __device__ __forceinline__ void expand_tail_ntt(const Dev4 &P, uint32_t galois, 
     l1[k] = add_mod<Q>(h1[k], n1v);
     const ulonglong2 lam =
         __ldg(P.T.pwt[L] + ((2 * kN - ((kshift * e) & (2 * kN - 1))) & (2 * kN - 1)));
-    const uint64_t t0 = mul_shoup<Q>(sub_mod<Q>(h0[k], n0v), lam.x, lam.y);
-    const uint64_t t1 = mul_shoup<Q>(sub_mod<Q>(h1[k], n1v), lam.x, lam.y);
+    const uint64_t t0 = opir60::mul<Q>(h0[k] - n0v + Q, lam);
+    const uint64_t t1 = opir60::mul<Q>(h1[k] - n1v + Q, lam);
     r0[k] = min(t0, t0 - Q);
     r1[k] = min(t1, t1 - Q);
   }
@@ -358,7 +358,7 @@ __device__ __forceinline__ void expand_body(const Dev4 &P, uint32_t galois_inv, 
         ulonglong2 wd[7];
         fload_d<L>(wd, P.T);
         ld_plane<3>(sm4 + e * kPad, v, tid);
-        fD<L>(v, wd);  // [0, 6q)
+        fD<L>(v, wd);
       }
       const uint64_t *R = key + static_cast<uint64_t>(i) * kRowWords + L * kN + 8 * tid;
       {
@@ -384,9 +384,9 @@ __device__ __forceinline__ void expand_body(const Dev4 &P, uint32_t galois_inv, 
     uint64_t vb[8], va[8];  // the key switch's delta in NTT form, canonical
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      vb[k] = fold16<Q>(ab[k]);
+      vb[k] = opir60::fold<Q>(ab[k]);
       vb[k] = min(vb[k], vb[k] - Q);
-      va[k] = fold16<Q>(aa[k]);
+      va[k] = opir60::fold<Q>(aa[k]);
       va[k] = min(va[k], va[k] - Q);
     }
     expand_tail_ntt<L>(P, galois, kshift, ct, vb, va, outL, outR);
@@ -397,7 +397,7 @@ __device__ __forceinline__ void expand_body(const Dev4 &P, uint32_t galois_inv, 
     iload_d<L>(wd, P.T);
     uint64_t vb[8], va[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) { vb[k] = fold16<Q>(ab[k]); va[k] = fold16<Q>(aa[k]); }
+    for (int k = 0; k < 8; ++k) { vb[k] = opir60::fold<Q>(ab[k]); va[k] = opir60::fold<Q>(aa[k]); }
     iD<L>(vb, wd);
     iD<L>(va, wd);
     st_plane<3>(sm4, vb, tid);
@@ -519,7 +519,7 @@ __device__ __forceinline__ void expand_split_body(const Dev4 &P, uint32_t galois
       ulonglong2 wd[7];
       fload_d<L>(wd, P.T);
       ld_plane<3>(sm4 + e * kPad, v, tid);
-      fD<L>(v, wd);  // [0, 6q)
+      fD<L>(v, wd);
     }
     const uint64_t *R = key + static_cast<uint64_t>(i) * kRowWords + L * kN + 8 * tid;
     {
@@ -563,7 +563,7 @@ __device__ __forceinline__ void expand_split_body(const Dev4 &P, uint32_t galois
     iload_d<L>(wd, P.T);
     uint64_t v[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = fold16<Q>(tot[k]);
+    for (int k = 0; k < 8; ++k) v[k] = opir60::fold<Q>(tot[k]);
     iD<L>(v, wd);
     st_plane<3>(sm4, v, tid);
   }
@@ -615,7 +615,7 @@ k4_expand_level_split(Dev4 P, uint32_t galois_inv, uint32_t kshift,
 // CRT-composed and split into l unsigned base-2^B digits; digit d of poly p
 // meets row p l + (l - 1 - d). Uses G planes (G = l when l <= 5, else 4).
 // Products are Shoup products in [0, 2q) with the rows' companions; the
-// sums are folded below 2q after each group (< 2q + 5 x 2q in between).
+// sums are folded after each group (q + 16 c + 5 x 2q in between).
 template <int L, int NL, int B>
 __device__ __forceinline__ void gadget_mac(const Dev4 &P, const uint64_t *x, const uint64_t *y,
                                            const uint64_t *rgsw, uint64_t *sm, uint64_t (&acc0)[8],
@@ -675,7 +675,7 @@ __device__ __forceinline__ void gadget_mac(const Dev4 &P, const uint64_t *x, con
         }
       }
 #pragma unroll
-      for (int k = 0; k < 8; ++k) { acc0[k] = fold16<Q>(acc0[k]); acc1[k] = fold16<Q>(acc1[k]); }
+      for (int k = 0; k < 8; ++k) { acc0[k] = opir60::fold<Q>(acc0[k]); acc1[k] = opir60::fold<Q>(acc1[k]); }
       __syncthreads();
     }
   }
@@ -728,7 +728,7 @@ __device__ __forceinline__ void selectors_body(const Dev4 &P, const Shape4 &S,
     fD<L>(v, wd);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const uint64_t c = canon8<Q>(v[k]);
+      const uint64_t c = opir60::canon<Q>(v[k]);
       top[p * 2 * kN + k] = c;
       top[4 * kN + p * 2 * kN + k] = shoup_of<Q>(c);
     }
@@ -786,9 +786,9 @@ __device__ __forceinline__ void fst_body(const Dev4 &P, const Shape4 &S, const u
     for (int h = 0; h < 2; ++h) {  // D-order positions 4 (tid + 512 h) .. + 3
       const int j0 = posD(tid, 4 * h);
       *reinterpret_cast<ulonglong2 *>(dst + j0) =
-          make_ulonglong2(canon8<Limb<L>::q>(v[4 * h + 0]), canon8<Limb<L>::q>(v[4 * h + 1]));
+          make_ulonglong2(opir60::canon<Limb<L>::q>(v[4 * h + 0]), opir60::canon<Limb<L>::q>(v[4 * h + 1]));
       *reinterpret_cast<ulonglong2 *>(dst + j0 + 2) =
-          make_ulonglong2(canon8<Limb<L>::q>(v[4 * h + 2]), canon8<Limb<L>::q>(v[4 * h + 3]));
+          make_ulonglong2(opir60::canon<Limb<L>::q>(v[4 * h + 2]), opir60::canon<Limb<L>::q>(v[4 * h + 3]));
     }
   }
 }
@@ -950,7 +950,7 @@ __device__ __forceinline__ void mux_body(const Dev4 &P, const Shape4 &S, uint32_
     iload_d<L>(wd, P.T);
     uint64_t v[8], w[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) { v[k] = acc0[k]; w[k] = acc1[k]; }  // [0, 2q)
+    for (int k = 0; k < 8; ++k) { v[k] = acc0[k]; w[k] = acc1[k]; }
     iD<L>(v, wd);
     iD<L>(w, wd);
     st_plane<3>(sm4, v, tid);
@@ -985,9 +985,9 @@ k4_mux_level(Dev4 P, Shape4 S, uint32_t level, uint32_t n_pairs, uint32_t offset
 // MUX level, cluster split: with fewer pairs than SMs each MUX runs on a
 // cluster of C CTAs. CTA r takes digits [d0, d0 + dn) of polynomial p of
 // y - x (C = 2: p = r, all l digits; C = 4: p = r / 2, digits 0-2 or 3-4),
-// accumulates their Shoup products with the RGSW rows and folds them below
-// 2q; CTAs 0 and 1 add the partials (below 2q C) through distributed shared
-// memory, fold them below 2q and finish output polynomial c0 / c1 (INTT,
+// accumulates their Shoup products with the RGSW rows and folds them; CTAs 0
+// and 1 add the partials through distributed shared memory, fold them and
+// finish output polynomial c0 / c1 (INTT,
 // + x). The same residues enter the same INTT: bit for bit the single-CTA
 // MUX.
 template <int L>
@@ -1041,7 +1041,7 @@ __device__ __forceinline__ void gadget_part(const Dev4 &P, const uint64_t *x, co
     }
   }
 #pragma unroll
-  for (int k = 0; k < 8; ++k) { acc0[k] = fold16<Q>(acc0[k]); acc1[k] = fold16<Q>(acc1[k]); }
+  for (int k = 0; k < 8; ++k) { acc0[k] = opir60::fold<Q>(acc0[k]); acc1[k] = opir60::fold<Q>(acc1[k]); }
   __syncthreads();
 }
 
@@ -1098,7 +1098,7 @@ __device__ __forceinline__ void mux_split_body(const Dev4 &P, const Shape4 &S, u
     iload_d<L>(wd, P.T);
     uint64_t v[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = fold16<Q>(tot[k]);  // < 2q C <= 8q -> [0, 2q)
+    for (int k = 0; k < 8; ++k) v[k] = opir60::fold<Q>(tot[k]);
     iD<L>(v, wd);
     st_plane<3>(sm4, v, tid);
   }
@@ -1178,28 +1178,21 @@ void note_launches(int64_t delta) {
   g_launches4.fetch_add(static_cast<uint64_t>(delta), std::memory_order_relaxed);
 }
 
-void upload_constants(const uint64_t *const fw[2], const uint64_t *const fw_sh[2],
-                      const uint64_t *const iw[2], const uint64_t *const iw_sh[2],
-                      const uint64_t ninv[2][2], const uint64_t w1ninv[2][2]) {
+void upload_constants(const ulonglong2 *const fw[2], const ulonglong2 *const iw[2],
+                      const ulonglong2 ninv[2], const ulonglong2 w1ninv[2]) {
   static std::mutex mu;
   static std::set<int> done;
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
   if (done.count(dev)) return;
-  ulonglong2 f[2][64], i[2][64], a[2], b[2];
-  for (int r = 0; r < 2; ++r) {
-    for (int k = 0; k < 64; ++k) {
-      f[r][k] = make_ulonglong2(fw[r][k], fw_sh[r][k]);
-      i[r][k] = make_ulonglong2(iw[r][k], iw_sh[r][k]);
-    }
-    a[r] = make_ulonglong2(ninv[r][0], ninv[r][1]);
-    b[r] = make_ulonglong2(w1ninv[r][0], w1ninv[r][1]);
+  cudaError_t e = cudaSuccess;
+  for (int r = 0; r < 2 && e == cudaSuccess; ++r) {
+    e = cudaMemcpyToSymbol(c4_fwt, fw[r], sizeof(c4_fwt[0]), r * sizeof(c4_fwt[0]));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(c4_iwt, iw[r], sizeof(c4_iwt[0]), r * sizeof(c4_iwt[0]));
   }
-  cudaError_t e = cudaMemcpyToSymbol(c4_fwt, f, sizeof(f));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c4_iwt, i, sizeof(i));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c4_ninv, a, sizeof(a));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c4_w1ninv, b, sizeof(b));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c4_ninv, ninv, sizeof(c4_ninv));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c4_w1ninv, w1ninv, sizeof(c4_w1ninv));
   if (e != cudaSuccess)
     throw std::runtime_error(std::string("NTT constants: ") + cudaGetErrorString(e));
   done.insert(dev);
@@ -1397,9 +1390,9 @@ void launch_modswitch(const Dev4 &P, const uint64_t *ct, uint64_t ct_stride, uin
 }
 
 // ------------------------------------------------- butterfly-rate probe
-// The two-limb NTT's forward radix-8 pass (fpass, limb 0) on register values
-// and twiddles, three passes per iteration with one pass's corrections per
-// stage pattern of the kernels; see the single-modulus probe.
+// The two-limb NTT's forward radix-8 pass (opir60::fpass8, limb 0) on
+// register values and twiddles, three passes per iteration; see the
+// single-modulus probe.
 __global__ void __launch_bounds__(256)
 k4_bfly_rate(uint64_t *__restrict__ sink, uint32_t iters, ulonglong2 w0) {
   uint64_t v[8];
@@ -1409,9 +1402,9 @@ k4_bfly_rate(uint64_t *__restrict__ sink, uint32_t iters, ulonglong2 w0) {
 #pragma unroll
   for (int k = 0; k < 7; ++k) w[k] = make_ulonglong2(w0.x + 2 * k, w0.y + k);
   for (uint32_t it = 0; it < iters; ++it) {
-    fpass<kQ0, false, false, false>(v, w);
-    fpass<kQ0, true, false, true>(v, w);
-    fpass<kQ0, false, true, false>(v, w);
+    opir60::fpass8<kQ0, true>(v, w);
+    opir60::fpass8<kQ0, false>(v, w);
+    opir60::fpass8<kQ0, false>(v, w);
   }
   uint64_t acc = 0;
 #pragma unroll
@@ -1427,9 +1420,7 @@ uint32_t bfly_rate_blocks(int sms) {
 }
 
 uint64_t launch_bfly_rate(uint64_t *sink, uint32_t blocks, uint32_t iters, cudaStream_t st) {
-  const uint64_t w = 1234567890123456789ull % kQ0;
-  const ulonglong2 w0 = make_ulonglong2(
-      w, static_cast<uint64_t>((static_cast<unsigned __int128>(w) << 64) / kQ0));
+  const ulonglong2 w0 = opir60::twiddle(1234567890123456789ull % kQ0, kQ0);
   k4_bfly_rate<<<blocks, 256, 0, st>>>(sink, iters, w0);
   check_launch("k4_bfly_rate");
   return static_cast<uint64_t>(blocks) * 256 * iters * 36;

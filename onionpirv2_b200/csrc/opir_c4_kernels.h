@@ -31,10 +31,10 @@ constexpr uint64_t kQ1 = 1152921504606748673ull;  // 2^60 - 2^16 - 2^15 + 1
 constexpr int kCtWords = 4 * kN;  // u64 words per ciphertext (2 polys x 2 limbs)
 constexpr int kRowWords = 8 * kN; // a key / RGSW row: ciphertext + Shoup companions
 
-// Full twiddle tables in global memory, (w, floor(w 2^64 / q)) pairs per limb
+// Full twiddle tables in global memory per limb (opir60::twiddle)
 struct Tables {
   const ulonglong2 *fwt[2], *iwt[2];
-  const ulonglong2 *pwt[2];  // (psi^m, floor(psi^m 2^64 / q)) for m < 2N
+  const ulonglong2 *pwt[2];  // psi^m for m < 2N
 };
 
 struct Dev4 {
@@ -54,9 +54,10 @@ uint64_t launch_count();
 // kernels replayed from a CUDA graph).
 void note_launches(int64_t delta);
 
-void upload_constants(const uint64_t *const fw[2], const uint64_t *const fw_sh[2],
-                      const uint64_t *const iw[2], const uint64_t *const iw_sh[2],
-                      const uint64_t ninv[2][2], const uint64_t w1ninv[2][2]);
+// Twiddles with index < 64, N^-1 and iw[1] N^-1 per limb (opir60::twiddle) to
+// the kernels' constant memory of the current device (once per device).
+void upload_constants(const ulonglong2 *const fw[2], const ulonglong2 *const iw[2],
+                      const ulonglong2 ninv[2], const ulonglong2 w1ninv[2]);
 
 // Nodes of expansion level d that lead to a useful leaf (server.cpp:794-809).
 uint32_t expand_nodes(const Shape4 &s, uint32_t d);

@@ -14,6 +14,7 @@
 #include <stdexcept>
 #include <string>
 
+#include "opir_fold60.cuh"
 #include "opir_k1p_kernels.h"
 #include "opir_params.h"
 #include "opir_scan_tc.h"
@@ -132,26 +133,25 @@ Server::Server(const opir_params &p, cudaStream_t stream, const opir::RowShard *
   ck(cudaStreamSynchronize(st_), "create");
 }
 
-// Twiddle tables of CONFIG_N2048_K1: [forward N][inverse N] (w, Shoup) of
+// Twiddle tables of CONFIG_N2048_K1: [forward N][inverse N] of
 // the one limb, the first 64 of each to constant memory.
 void Server::setup_k1_tables() {
   const opir::LimbTables64 t = opir::make_limb_tables64(n_, p_.q, p_.w1);
-  // [forward N][inverse N] (w, Shoup) pairs, then (psi^m, Shoup) for m < 2N
+  // [forward N][inverse N] (opir60::twiddle), then psi^m for m < 2N
   std::vector<ulonglong2> host(4ull * n_);
   for (uint32_t i = 0; i < n_; ++i) {
-    host[i] = make_ulonglong2(t.fw[i], t.fw_sh[i]);
-    host[n_ + i] = make_ulonglong2(t.iw[i], t.iw_sh[i]);
+    host[i] = opir60::twiddle(t.fw[i], t.q);
+    host[n_ + i] = opir60::twiddle(t.iw[i], t.q);
   }
   {
     // psi = fw[brev(1)] = fw[N / 2] (fw[k] = psi^brev(k))
     const uint64_t q = t.q, psi = t.fw[n_ / 2];
     uint64_t pw = 1;
     for (uint32_t m = 0; m < 2 * n_; ++m) {
-      const uint64_t sh = static_cast<uint64_t>((static_cast<unsigned __int128>(pw) << 64) / q);
-      host[2 * n_ + m] = make_ulonglong2(pw, sh);
+      host[2 * n_ + m] = opir60::twiddle(pw, q);
       pw = static_cast<uint64_t>(static_cast<unsigned __int128>(pw) * psi % q);
     }
-    if (pw != 1 || host[2 * n_ + n_].x != q - 1)
+    if (pw != 1 || host[2 * n_ + n_].x != opir60::twiddle(q - 1, q).x)
       throw std::runtime_error("psi is not a primitive 2N-th root of unity");
   }
   tables_.alloc(host.size());
@@ -160,8 +160,8 @@ void Server::setup_k1_tables() {
   dp_.T.fwt[0] = dp_.T.fwt[1] = tables_.p;
   dp_.T.iwt[0] = dp_.T.iwt[1] = tables_.p + n_;
   dp_.T.pwt[0] = dp_.T.pwt[1] = tables_.p + 2 * n_;
-  const uint64_t ninv[2] = {t.n_inv, t.n_inv_sh}, w1n[2] = {t.w1_ninv, t.w1_ninv_sh};
-  opir1::upload_constants(t.fw.data(), t.fw_sh.data(), t.iw.data(), t.iw_sh.data(), ninv, w1n);
+  const ulonglong2 scale[2] = {opir60::twiddle(t.n_inv, t.q), opir60::twiddle(t.w1_ninv, t.q)};
+  opir1::upload_constants(host.data(), host.data() + n_, scale);
 }
 
 opir1::Dev1 Server::d1() const {
@@ -173,22 +173,21 @@ void Server::setup_c4_tables() {
   const opir::LimbTables64 t[2] = {opir::make_limb_tables64(kN, p_.q1, p_.w1),
                                    opir::make_limb_tables64(kN, p_.q2, p_.w2)};
   if (t[0].q != kQ0 || t[1].q != kQ1) throw std::invalid_argument("unexpected RNS limbs");
-  // [limb][forward N][inverse N] (w, Shoup) pairs, then [limb][psi^m, m < 2N]
+  // [limb][forward N][inverse N] (opir60::twiddle), then [limb][psi^m, m < 2N]
   std::vector<ulonglong2> host(8ull * kN);
   for (int l = 0; l < 2; ++l) {
     for (int i = 0; i < kN; ++i) {
-      host[l * 2 * kN + i] = make_ulonglong2(t[l].fw[i], t[l].fw_sh[i]);
-      host[l * 2 * kN + kN + i] = make_ulonglong2(t[l].iw[i], t[l].iw_sh[i]);
+      host[l * 2 * kN + i] = opir60::twiddle(t[l].fw[i], t[l].q);
+      host[l * 2 * kN + kN + i] = opir60::twiddle(t[l].iw[i], t[l].q);
     }
     // psi = fw[brev(1)] = fw[N / 2] (fw[k] = psi^brev(k))
     const uint64_t q = t[l].q, psi = t[l].fw[kN / 2];
     uint64_t pw = 1;
     for (int m = 0; m < 2 * kN; ++m) {
-      const uint64_t sh = static_cast<uint64_t>((static_cast<unsigned __int128>(pw) << 64) / q);
-      host[4 * kN + l * 2 * kN + m] = make_ulonglong2(pw, sh);
+      host[4 * kN + l * 2 * kN + m] = opir60::twiddle(pw, q);
       pw = static_cast<uint64_t>(static_cast<unsigned __int128>(pw) * psi % q);
     }
-    if (pw != 1 || host[4 * kN + l * 2 * kN + kN].x != q - 1)
+    if (pw != 1 || host[4 * kN + l * 2 * kN + kN].x != opir60::twiddle(q - 1, q).x)
       throw std::runtime_error("psi is not a primitive 2N-th root of unity");
   }
   tables_.alloc(host.size());
@@ -199,13 +198,11 @@ void Server::setup_c4_tables() {
     dp_.T.iwt[l] = tables_.p + l * 2 * kN + kN;
     dp_.T.pwt[l] = tables_.p + 4 * kN + l * 2 * kN;
   }
-  const uint64_t *fw[2] = {t[0].fw.data(), t[1].fw.data()};
-  const uint64_t *fw_sh[2] = {t[0].fw_sh.data(), t[1].fw_sh.data()};
-  const uint64_t *iw[2] = {t[0].iw.data(), t[1].iw.data()};
-  const uint64_t *iw_sh[2] = {t[0].iw_sh.data(), t[1].iw_sh.data()};
-  const uint64_t ninv[2][2] = {{t[0].n_inv, t[0].n_inv_sh}, {t[1].n_inv, t[1].n_inv_sh}};
-  const uint64_t w1n[2][2] = {{t[0].w1_ninv, t[0].w1_ninv_sh}, {t[1].w1_ninv, t[1].w1_ninv_sh}};
-  upload_constants(fw, fw_sh, iw, iw_sh, ninv, w1n);
+  const ulonglong2 *fw[2] = {host.data(), host.data() + 2 * kN};
+  const ulonglong2 *iw[2] = {host.data() + kN, host.data() + 3 * kN};
+  const ulonglong2 ninv[2] = {opir60::twiddle(t[0].n_inv, t[0].q), opir60::twiddle(t[1].n_inv, t[1].q)};
+  const ulonglong2 w1n[2] = {opir60::twiddle(t[0].w1_ninv, t[0].q), opir60::twiddle(t[1].w1_ninv, t[1].q)};
+  upload_constants(fw, iw, ninv, w1n);
   dp_.q0inv = p_.q1_inv_mod_q2;
   dp_.q0inv_sh = static_cast<uint64_t>((static_cast<unsigned __int128>(dp_.q0inv) << 64) / kQ1);
 }

@@ -3,14 +3,16 @@
 //
 // NTT: the register-resident radix-8/8/8/4 form of the CONFIG_N2048_K1_COMP
 // kernels (opir_device.cuh: 256 threads x 8 coefficients, thread positions
-// A/B/C/D, shared planes padded by one word per 32) in 64-bit arithmetic:
-// Harvey/Shoup lazy butterflies with w' = floor(w 2^64 / q), forward values
-// below 8q < 2^63 with X corrected on stages 4, 6, 8 and 10, inverse values
-// in [0, 2q). Merged Cooley-Tukey forward with bit-reversed output,
-// Gentleman-Sande inverse scaled by N^-1 (the HEXL convention the reference
-// registers, utils.cpp:26-56). Key and selector rows carry Shoup companions,
-// so every key product is three 64-bit multiplies landing in [0, 2q).
+// A/B/C/D, shared planes padded by one word per 32) in 64-bit arithmetic
+// that folds modulo q = 2^60 - c (opir_fold60.cuh): forward values grow by
+// about q a stage and stay below 2^64, inverse passes begin and end folded.
+// Merged Cooley-Tukey forward with bit-reversed output, Gentleman-Sande
+// inverse scaled by N^-1 (the HEXL convention the reference registers,
+// utils.cpp:26-56). Key and selector rows carry Shoup companions, so every
+// key product is three 64-bit multiplies landing in [0, 2q).
 #include "opir_k1p_kernels.h"
+
+#include "opir_fold60.cuh"
 
 #include <map>
 #include <mutex>
@@ -28,8 +30,8 @@ constexpr int kThreads = 256;
 constexpr int kPad = kN + kN / 32;  // u64 words per padded plane
 constexpr uint64_t kGolden = 0x9E3779B97F4A7C15ull;
 
-// (w, Shoup) for twiddle indices < 64, forward and inverse; {N^-1, its
-// Shoup companion} and {iw[1] N^-1, Shoup}
+// opir60::twiddle() of the twiddles with index < 64, forward and inverse, and
+// of N^-1 and iw[1] N^-1
 static __constant__ ulonglong2 c1_fwt[64];
 static __constant__ ulonglong2 c1_iwt[64];
 static __constant__ ulonglong2 c1_nscale[2];
@@ -87,11 +89,6 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {  // splitmix64 finaliser
 __device__ __forceinline__ uint64_t mulsh(uint64_t a, uint64_t w, uint64_t ws) {
   return a * w - __umul64hi(a, ws) * kQ;
 }
-__device__ __forceinline__ uint64_t canon8(uint64_t x) {  // [0, 8q) -> [0, q)
-  x = min(x, x - 4 * kQ);
-  x = min(x, x - 2 * kQ);
-  return min(x, x - kQ);
-}
 __device__ __forceinline__ uint64_t fold2(uint64_t x) { return min(x, x - kQ); }  // [0, 2q)
 __device__ __forceinline__ uint64_t add_q(uint64_t a, uint64_t b) {
   const uint64_t s = a + b;
@@ -148,28 +145,11 @@ __device__ __forceinline__ void ld_plane(const uint64_t *pl, uint64_t (&v)[8], i
   }
 }
 
-template <bool C>
-__device__ __forceinline__ void fbf(uint64_t &X, uint64_t &Y, ulonglong2 w) {
-  uint64_t x = X;
-  if (C) x = min(x, x - 4 * kQ);
-  const uint64_t t = mulsh(Y, w.x, w.y);
-  X = x + t;
-  Y = x - t + 2 * kQ;
-}
-template <bool C1, bool C2, bool C3>
-__device__ __forceinline__ void fpass8(uint64_t (&v)[8], const ulonglong2 (&w)[7]) {
-  fbf<C1>(v[0], v[4], w[0]); fbf<C1>(v[1], v[5], w[0]);
-  fbf<C1>(v[2], v[6], w[0]); fbf<C1>(v[3], v[7], w[0]);
-  fbf<C2>(v[0], v[2], w[1]); fbf<C2>(v[1], v[3], w[1]);
-  fbf<C2>(v[4], v[6], w[2]); fbf<C2>(v[5], v[7], w[2]);
-  fbf<C3>(v[0], v[1], w[3]); fbf<C3>(v[2], v[3], w[4]);
-  fbf<C3>(v[4], v[5], w[5]); fbf<C3>(v[6], v[7], w[6]);
-}
 // pass A (stages 1-3), canonical input
 __device__ __forceinline__ void fA(uint64_t (&v)[8]) {
   const ulonglong2 w[7] = {c1_fwt[1], c1_fwt[2], c1_fwt[3], c1_fwt[4],
                            c1_fwt[5], c1_fwt[6], c1_fwt[7]};
-  fpass8<false, false, false>(v, w);
+  opir60::fpass8<kQ, true>(v, w);
 }
 __device__ __forceinline__ void load_b(ulonglong2 (&w)[7], const ulonglong2 *c, int t) {
   const int g = t >> 5;
@@ -196,32 +176,27 @@ __device__ __forceinline__ void load_d(ulonglong2 (&w)[6], const ulonglong2 *tw,
     w[3 * h + 2] = __ldg(tw + 1025 + 2 * b4);
   }
 }
-// pass D (stages 10-11): output in [0, 8q)
+// pass D (stages 10-11): output any 64 bits
 __device__ __forceinline__ void fD(uint64_t (&v)[8], const ulonglong2 (&w)[6]) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     uint64_t *u = v + 4 * h;
-    fbf<true>(u[0], u[2], w[3 * h]);
-    fbf<true>(u[1], u[3], w[3 * h]);
-    fbf<false>(u[0], u[1], w[3 * h + 1]);
-    fbf<false>(u[2], u[3], w[3 * h + 2]);
+    opir60::fbf<kQ>(u[0], u[2], w[3 * h]);
+    opir60::fbf<kQ>(u[1], u[3], w[3 * h]);
+    opir60::fbf<kQ>(u[0], u[1], w[3 * h + 1]);
+    opir60::fbf<kQ>(u[2], u[3], w[3 * h + 2]);
   }
 }
 // passes B and C over np planes stored in A-order after fA (up to a
 // __syncthreads); ends synchronised. Full = true unrolls the plane loops
 // (faster in the expansion and MUX levels; the selector kernel keeps the
 // compiler's choice, which is faster there).
-__device__ __forceinline__ void ipass8(uint64_t (&v)[8], const ulonglong2 (&w)[7]);
 template <int PASS, bool FWD>
 __device__ __forceinline__ void mid_plane(uint64_t *pl, const ulonglong2 (&w)[7], int t) {
   uint64_t v[8];
   ld_plane<PASS>(pl, v, t);
-  if (FWD) {
-    if (PASS == 1) fpass8<true, false, true>(v, w);
-    else fpass8<false, true, false>(v, w);
-  } else {
-    ipass8(v, w);
-  }
+  if (FWD) opir60::fpass8<kQ, false>(v, w);
+  else opir60::ipass8<kQ>(v, w);
   st_plane<PASS>(pl, v, t);
 }
 template <bool Full = true>
@@ -251,30 +226,14 @@ __device__ __forceinline__ void fwd_mid(uint64_t *sm, int np, const ulonglong2 *
   __syncthreads();
 }
 
-__device__ __forceinline__ void ibf(uint64_t &X, uint64_t &Y, ulonglong2 w) {
-  uint64_t u = X + Y;
-  u = min(u, u - 2 * kQ);
-  const uint64_t d = X - Y + 2 * kQ;
-  Y = mulsh(d, w.x, w.y);
-  X = u;
-}
-__device__ __forceinline__ void ipass8(uint64_t (&v)[8], const ulonglong2 (&w)[7]) {
-  ibf(v[0], v[1], w[3]); ibf(v[2], v[3], w[4]);
-  ibf(v[4], v[5], w[5]); ibf(v[6], v[7], w[6]);
-  ibf(v[0], v[2], w[1]); ibf(v[1], v[3], w[1]);
-  ibf(v[4], v[6], w[2]); ibf(v[5], v[7], w[2]);
-  ibf(v[0], v[4], w[0]); ibf(v[1], v[5], w[0]);
-  ibf(v[2], v[6], w[0]); ibf(v[3], v[7], w[0]);
-}
-// first inverse pass (stages t = 1, 2) on D-order values in [0, 2q)
+// first inverse pass (stages t = 1, 2) on folded D-order values
 __device__ __forceinline__ void iD(uint64_t (&v)[8], const ulonglong2 (&w)[6]) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     uint64_t *u = v + 4 * h;
-    ibf(u[0], u[1], w[3 * h + 1]);
-    ibf(u[2], u[3], w[3 * h + 2]);
-    ibf(u[0], u[2], w[3 * h]);
-    ibf(u[1], u[3], w[3 * h]);
+    opir60::ipass4<kQ>(u[0], u[1], u[2], u[3], w[3 * h + 1], w[3 * h + 2], w[3 * h]);
+    u[0] = opir60::fold<kQ>(u[0]);
+    u[1] = opir60::fold<kQ>(u[1]);
   }
 }
 // passes C and B over np planes holding D-order values after iD (up to a
@@ -307,17 +266,7 @@ __device__ __forceinline__ void inv_mid(uint64_t *sm, int np, const ulonglong2 *
 }
 // last inverse pass (t = 256, 512, then 1024 with N^-1 folded in); canonical
 __device__ __forceinline__ void iA(uint64_t (&v)[8]) {
-  ibf(v[0], v[1], c1_iwt[4]); ibf(v[2], v[3], c1_iwt[5]);
-  ibf(v[4], v[5], c1_iwt[6]); ibf(v[6], v[7], c1_iwt[7]);
-  ibf(v[0], v[2], c1_iwt[2]); ibf(v[1], v[3], c1_iwt[2]);
-  ibf(v[4], v[6], c1_iwt[3]); ibf(v[5], v[7], c1_iwt[3]);
-  const ulonglong2 ni = c1_nscale[0], wn = c1_nscale[1];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint64_t X = v[k], Y = v[k + 4];
-    v[k] = fold2(mulsh(X + Y, ni.x, ni.y));
-    v[k + 4] = fold2(mulsh(X - Y + 2 * kQ, wn.x, wn.y));
-  }
+  opir60::ilast8<kQ>(v, c1_iwt, c1_nscale[0], c1_nscale[1]);
 }
 
 // Four consecutive u64 of a row at D-order positions 4 (t + 256 h) .. + 3.
@@ -340,14 +289,6 @@ __device__ __forceinline__ void mac_part(const uint64_t *row, int part, const ui
     for (int m = 0; m < 4; ++m) acc[4 * h + m] += mulsh(v[4 * h + m], w[m], ws[m]);
   }
 }
-// [0, 2q G) -> [0, 2q) for the running sums (G <= 7 products of [0, 2q)
-// plus a folded sum, below 16q < 2^64)
-__device__ __forceinline__ uint64_t fold16(uint64_t x) {
-  x = min(x, x - 8 * kQ);
-  x = min(x, x - 4 * kQ);
-  return min(x, x - 2 * kQ);
-}
-
 // ------------------------------------------------------------ DB preprocessing
 // server.cpp:80-203 with one prime: pt mod q, NTT, the coefficient-major
 // transpose as eight byte planes per NTT level, db8[(z 8 + plane)][row][n0p].
@@ -384,7 +325,7 @@ k1p_db_preprocess(Dev1 P, const uint64_t *__restrict__ coeffs, uint64_t coeff_pt
     ld_plane<3>(sm1 + e * kPad, out[e], tid);
     fD(out[e], wd);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) out[e][k] = canon8(out[e][k]);
+    for (int k = 0; k < 8; ++k) out[e][k] = opir60::canon<kQ>(out[e][k]);
   }
   const uint64_t row = pt0 / n0, col = pt0 % n0;
   const uint64_t pb = static_cast<uint64_t>(other) * n0p;  // bytes per plane
@@ -421,7 +362,7 @@ k1p_db_preprocess(Dev1 P, const uint64_t *__restrict__ coeffs, uint64_t coeff_pt
 // One heap node per CTA: the BV key switch (bv_keyswitch.cpp:296-367) of the
 // node and its two children (server.cpp:794-809): left = c + c', right =
 // (c - c') X^-k, sigma_k(c)[j] = +-c[j k^-1 mod 2N]. Digits in groups of 4
-// planes; Shoup key products summed below 2q after each group.
+// planes; sums of Shoup key products folded after each group.
 constexpr int kGroup = 4;
 
 // Children of the last level in NTT form (the first-dimension leaves), from
@@ -459,8 +400,8 @@ __device__ __forceinline__ void expand_tail_ntt(const Dev1 &P, uint32_t galois, 
   }
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
-    h0[k] = canon8(h0[k]);
-    h1[k] = canon8(h1[k]);
+    h0[k] = opir60::canon<kQ>(h0[k]);
+    h1[k] = opir60::canon<kQ>(h1[k]);
   }
   st_plane<3>(sm1 + 2 * kPad, h0, tid);  // c0^ by slot, for the sigma gather
   __syncthreads();
@@ -478,8 +419,8 @@ __device__ __forceinline__ void expand_tail_ntt(const Dev1 &P, uint32_t galois, 
       l1[c] = add_q(h1[k], n1v);
       const ulonglong2 lam =
           __ldg(P.pwt + ((2 * kN - ((kshift * e) & (2 * kN - 1))) & (2 * kN - 1)));
-      r0[c] = fold2(mulsh(sub_q(h0[k], n0v), lam.x, lam.y));
-      r1[c] = fold2(mulsh(sub_q(h1[k], n1v), lam.x, lam.y));
+      r0[c] = fold2(opir60::mul<kQ>(h0[k] - n0v + kQ, lam));
+      r1[c] = fold2(opir60::mul<kQ>(h1[k] - n1v + kQ, lam));
     }
     const int j0 = posD(tid, 4 * h);  // four consecutive slots
     *reinterpret_cast<ulonglong2 *>(outL + j0) = make_ulonglong2(l0[0], l0[1]);
@@ -537,7 +478,7 @@ __device__ __forceinline__ void expand_body(const Dev1 &P, uint32_t galois_inv, 
       mac_part(R, 1, v, aa, tid);
     }
 #pragma unroll
-    for (int k = 0; k < 8; ++k) { ab[k] = fold16(ab[k]); aa[k] = fold16(aa[k]); }
+    for (int k = 0; k < 8; ++k) { ab[k] = opir60::fold<kQ>(ab[k]); aa[k] = opir60::fold<kQ>(aa[k]); }
     __syncthreads();
   }
   uint64_t *outL = out + (static_cast<uint64_t>(b) * out_stride + 2ull * node) * kCtWords;
@@ -555,7 +496,7 @@ __device__ __forceinline__ void expand_body(const Dev1 &P, uint32_t galois_inv, 
   {
     ulonglong2 wd[6];
     load_d(wd, P.iwt, tid);
-    iD(ab, wd);  // [0, 2q) in
+    iD(ab, wd);
     iD(aa, wd);
     st_plane<3>(sm1, ab, tid);
     st_plane<3>(sm1 + kPad, aa, tid);
@@ -614,7 +555,7 @@ k1p_expand_level_ntt(Dev1 P, uint32_t galois, uint32_t galois_inv, uint32_t kshi
 // each polynomial p of the decomposed ciphertext (y - x, or x when y is
 // null) split into L balanced base-2^B digits; digit d of poly p meets row
 // p L + (L - 1 - d) (MSB-first rows). Digit planes in groups of up to 5;
-// sums folded below 2q after each group.
+// sums folded after each group.
 template <int L, int B, bool Full = true>
 __device__ __forceinline__ void gadget_mac(const Dev1 &P, const uint64_t *x, const uint64_t *y,
                                            const uint64_t *rgsw, uint64_t *sm,
@@ -656,7 +597,7 @@ __device__ __forceinline__ void gadget_mac(const Dev1 &P, const uint64_t *x, con
         mac_part(R, 1, v, acc1, tid);
       }
 #pragma unroll
-      for (int k = 0; k < 8; ++k) { acc0[k] = fold16(acc0[k]); acc1[k] = fold16(acc1[k]); }
+      for (int k = 0; k < 8; ++k) { acc0[k] = opir60::fold<kQ>(acc0[k]); acc1[k] = opir60::fold<kQ>(acc1[k]); }
       __syncthreads();
     }
   }
@@ -710,7 +651,7 @@ k1p_selectors(Dev1 P, Shape1 S, const uint64_t *__restrict__ leaves, uint64_t le
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int j = posD(tid, k);
-      const uint64_t c = canon8(v[k]);
+      const uint64_t c = opir60::canon<kQ>(v[k]);
       top[p * kN + j] = c;
       top[2 * kN + p * kN + j] = shoup_of(c);
     }
@@ -755,9 +696,9 @@ k1p_fst_ntt(Dev1 P, Shape1 S, const uint64_t *__restrict__ leaves, uint64_t leaf
     for (int h = 0; h < 2; ++h) {  // D-order positions 4 (tid + 256 h) .. + 3
       const int j0 = posD(tid, 4 * h);
       *reinterpret_cast<ulonglong2 *>(dst + j0) =
-          make_ulonglong2(canon8(v[4 * h + 0]), canon8(v[4 * h + 1]));
+          make_ulonglong2(opir60::canon<kQ>(v[4 * h + 0]), opir60::canon<kQ>(v[4 * h + 1]));
       *reinterpret_cast<ulonglong2 *>(dst + j0 + 2) =
-          make_ulonglong2(canon8(v[4 * h + 2]), canon8(v[4 * h + 3]));
+          make_ulonglong2(opir60::canon<kQ>(v[4 * h + 2]), opir60::canon<kQ>(v[4 * h + 3]));
     }
   }
 }
@@ -883,7 +824,7 @@ k1p_mux_level(Dev1 P, Shape1 S, uint32_t level, uint32_t n_pairs, uint32_t offse
   {
     ulonglong2 wd[6];
     load_d(wd, P.iwt, tid);
-    iD(acc0, wd);  // [0, 2q) in
+    iD(acc0, wd);
     iD(acc1, wd);
     st_plane<3>(sm1, acc0, tid);
     st_plane<3>(sm1 + kPad, acc1, tid);
@@ -946,24 +887,16 @@ k1p_modswitch(Dev1 P, const uint64_t *__restrict__ ct_all, uint64_t ct_stride,
 }  // namespace
 
 // ===================================================================== launchers
-void upload_constants(const uint64_t *fw, const uint64_t *fw_sh, const uint64_t *iw,
-                      const uint64_t *iw_sh, const uint64_t ninv[2], const uint64_t w1ninv[2]) {
+void upload_constants(const ulonglong2 *fw, const ulonglong2 *iw, const ulonglong2 scale[2]) {
   static std::mutex mu;
   static std::set<int> done;
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
   if (done.count(dev)) return;
-  ulonglong2 f[64], i[64], sc[2];
-  for (int k = 0; k < 64; ++k) {
-    f[k] = make_ulonglong2(fw[k], fw_sh[k]);
-    i[k] = make_ulonglong2(iw[k], iw_sh[k]);
-  }
-  sc[0] = make_ulonglong2(ninv[0], ninv[1]);
-  sc[1] = make_ulonglong2(w1ninv[0], w1ninv[1]);
-  cudaError_t e = cudaMemcpyToSymbol(c1_fwt, f, sizeof(f));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c1_iwt, i, sizeof(i));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c1_nscale, sc, sizeof(sc));
+  cudaError_t e = cudaMemcpyToSymbol(c1_fwt, fw, sizeof(c1_fwt));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c1_iwt, iw, sizeof(c1_iwt));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c1_nscale, scale, sizeof(c1_nscale));
   if (e != cudaSuccess)
     throw std::runtime_error(std::string("CONFIG_N2048_K1 NTT constants: ") + cudaGetErrorString(e));
   done.insert(dev);

@@ -40,20 +40,19 @@ constexpr int kRowWords = 4 * kN;  // a key / RGSW row: ciphertext + Shoup compa
 constexpr int kLEp = 5, kBaseEp = 12, kLKey = 8, kBaseKey = 8, kLKs = 8, kBaseKs = 8;
 
 struct Dev1 {
-  const ulonglong2 *fwt, *iwt;  // (w, floor(w 2^64 / q)), bit-reversed order
+  const ulonglong2 *fwt, *iwt;  // opir60::twiddle, bit-reversed order
   uint64_t small_q;
   uint32_t small_q_width;
-  const ulonglong2 *pwt;        // (psi^m, floor(psi^m 2^64 / q)) for m < 2N
+  const ulonglong2 *pwt;        // psi^m for m < 2N
 };
 
 // the layout fields the kernels read (the two-limb set's shape struct)
 using Shape1 = opir4::Shape4;
 static_assert(kQ == opir4::kQ0, "the scan reduces CONFIG_N2048_K1 levels mod limb 0's prime");
 
-// Twiddles with index < 64 and {N^-1, iw[1] N^-1} (value, Shoup) to the
+// Twiddles with index < 64 and {N^-1, iw[1] N^-1} (opir60::twiddle) to the
 // kernels' constant memory of the current device (once per device).
-void upload_constants(const uint64_t *fw, const uint64_t *fw_sh, const uint64_t *iw,
-                      const uint64_t *iw_sh, const uint64_t ninv[2], const uint64_t w1ninv[2]);
+void upload_constants(const ulonglong2 *fw, const ulonglong2 *iw, const ulonglong2 scale[2]);
 
 // server.cpp:80-203: plaintexts [pt_begin, pt_end) -> NTT mod q -> db8.
 // coeffs (device, u64 < t) holds plaintexts from coeff_pt_begin on; null
