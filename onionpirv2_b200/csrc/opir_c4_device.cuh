@@ -46,8 +46,7 @@ __device__ __forceinline__ int posB(int t, int k) { return ((t >> 6) << 9) + (t 
 __device__ __forceinline__ int posC(int t, int k) { return ((t >> 3) << 6) + (t & 7) + 8 * k; }
 __device__ __forceinline__ int posD(int t, int k) { return 8 * t + k; }
 
-// a w mod q in [0, 2q) for any 64-bit a (Shoup; ws = floor(w 2^64 / q)): the
-// key rows, which carry that companion
+// a w mod q in [0, 2q) for any 64-bit a (Shoup; ws = floor(w 2^64 / q))
 template <uint64_t Q>
 __device__ __forceinline__ uint64_t mul_shoup(uint64_t a, uint64_t w, uint64_t ws) {
   return a * w - __umul64hi(a, ws) * Q;
@@ -212,19 +211,6 @@ __device__ __forceinline__ void iA(uint64_t (&v)[8]) {
   opir60::ilast8<Limb<L>::q>(v, c4_iwt[L], c4_ninv[L], c4_w1ninv[L]);
 }
 
-// floor(w 2^64 / q) for w < q = 2^60 - c: w 2^64 = w (16 q + 16 c), so the
-// quotient is 16 w + floor(x / q) with x = 16 c w < 2^81, and floor(x / q) is
-// t0 = floor(x / 2^60) or t0 + 1 (x / q - x / 2^60 < 2^-22); the remainder
-// x - t0 q = (x mod 2^60) + t0 c decides.
-template <uint64_t Q>
-__device__ __forceinline__ uint64_t shoup_of(uint64_t w) {
-  constexpr uint64_t c = (1ull << 60) - Q;
-  const unsigned __int128 x = static_cast<unsigned __int128>(w) * (16 * c);
-  const uint64_t hi = static_cast<uint64_t>(x >> 64), lo = static_cast<uint64_t>(x);
-  const uint64_t t0 = (hi << 4) | (lo >> 60);
-  const uint64_t r0 = (lo & ((1ull << 60) - 1)) + t0 * c;
-  return 16 * w + t0 + (r0 >= Q ? 1 : 0);
-}
 // ------------------------------------------------------ RNS <-> integer
 // Garner compose of canonical limbs into [0, q0 q1) (gsw.cpp:22-53)
 __device__ __forceinline__ unsigned __int128 compose(uint64_t r0, uint64_t r1, uint64_t q0inv,

@@ -125,6 +125,51 @@ __device__ __forceinline__ void ld8(const uint64_t *p, uint64_t (&v)[8]) {
   }
 }
 
+// One output polynomial of a group of np <= 5 digit planes (limb L): acc +=
+// sum of v_e x row e, rows `stride` words apart from R on; acc folded on entry
+// and exit. First runs pass D of the planes and leaves the transformed digits
+// in them as limbs.
+template <int L, bool First>
+__device__ __forceinline__ void mac_planes(const Dev4 &P, uint64_t *sm, int np, const uint64_t *R,
+                                           int64_t stride, uint64_t (&acc)[8]) {
+  constexpr uint64_t Q = Limb<L>::q;
+  const int tid = threadIdx.x;
+  uint64_t hi[8], mix[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) { hi[k] = 0; mix[k] = acc[k]; }
+#pragma unroll 1
+  for (int e = 0; e < np; ++e, R += stride) {
+    uint64_t w[8];
+    ld8(R, w);  // ahead of pass D
+    uint64_t v[8];
+    ld_plane<3>(sm + e * kPad, v, tid);
+    if constexpr (First) {
+      ulonglong2 wd[7];
+      fload_d<L>(wd, P.T);
+      fD<L>(v, wd);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = opir60::limbs<Q>(v[k]);
+      st_plane<3>(sm + e * kPad, v, tid);  // a thread's own eight slots
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) opir60::mac(acc[k], hi[k], mix[k], v[k], w[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) acc[k] = opir60::mac_join<Q>(acc[k], hi[k], mix[k]);
+}
+// acc0 / acc1 += sum over np planes of NTT(plane e) x row e's polynomial 0 / 1.
+// One output after the other: three 64-bit sums a coefficient for both at once
+// would be 96 of the 128 registers. Batch 8 of 2^18 entries: 14.78 ms; both
+// outputs at once on two sums a coefficient and a companion word per row word
+// 15.65 (the row loads wait behind pass D), Shoup products 15.20.
+template <int L>
+__device__ __forceinline__ void mac_group(const Dev4 &P, uint64_t *sm, int np, const uint64_t *row,
+                                          int64_t stride, uint64_t (&acc0)[8], uint64_t (&acc1)[8]) {
+  const uint64_t *R = row + L * kN + 8 * threadIdx.x;
+  mac_planes<L, true>(P, sm, np, R, stride, acc0);
+  mac_planes<L, false>(P, sm, np, R + 2 * kN, stride, acc1);
+}
+
 // ------------------------------------------------------------ gadget digits
 // Balanced BV digits (bv_keyswitch.cpp:42-62) lie in (-B/2, B/2]: the
 // centred value plus C = (B/2 - 1) sum_i B^i has plain base-B digits
@@ -237,8 +282,7 @@ k4_db_preprocess(Dev4 P, const uint64_t *__restrict__ coeffs, uint64_t coeff_pt_
 // One heap node, one limb per CTA: the K = 2 BV key switch of the node
 // (bv_keyswitch.cpp:373-481) and its two children (server.cpp:794-809).
 // Digits come from the CRT composition of sigma_k(c1) over both limbs. Key
-// products are Shoup products in [0, 2q) with the rows' stored companions,
-// so eight rows sum below 16q in 64 bits.
+// products accumulate in 30-bit limbs, two groups of four rows (mac_group).
 constexpr int kExpGroup = 4;  // digit planes per group
 
 // Children of the last level in NTT form (the first-dimension leaves), from
@@ -321,7 +365,7 @@ __device__ __forceinline__ void expand_body(const Dev4 &P, uint32_t galois_inv, 
   constexpr uint64_t Q = Limb<L>::q;
   const int node = node0 + blockIdx.x, b = blockIdx.z, tid = threadIdx.x;
   const uint64_t *ct = in + (static_cast<uint64_t>(b) * in_stride + node) * kCtWords;
-  const uint64_t *key = bv_keys[b] + bv_level_off;  // [row][b][a][b'][a']
+  const uint64_t *key = bv_keys[b] + bv_level_off;  // [row][b][a]
   uint64_t ab[8], aa[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) ab[k] = aa[k] = 0;
@@ -351,31 +395,8 @@ __device__ __forceinline__ void expand_body(const Dev4 &P, uint32_t galois_inv, 
     }
     __syncthreads();
     fwd_mid<L>(sm4, kExpGroup, P.T);
-    for (int e = 0; e < kExpGroup; ++e) {
-      const int i = g * kExpGroup + e;
-      uint64_t v[8];
-      {
-        ulonglong2 wd[7];
-        fload_d<L>(wd, P.T);
-        ld_plane<3>(sm4 + e * kPad, v, tid);
-        fD<L>(v, wd);
-      }
-      const uint64_t *R = key + static_cast<uint64_t>(i) * kRowWords + L * kN + 8 * tid;
-      {
-        uint64_t w[8], ws[8];
-        ld8(R, w);
-        ld8(R + 4 * kN, ws);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) ab[k] += mul_shoup<Q>(v[k], w[k], ws[k]);
-      }
-      {
-        uint64_t w[8], ws[8];
-        ld8(R + 2 * kN, w);
-        ld8(R + 6 * kN, ws);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) aa[k] += mul_shoup<Q>(v[k], w[k], ws[k]);
-      }
-    }
+    mac_group<L>(P, sm4, kExpGroup, key + static_cast<uint64_t>(g) * kExpGroup * kCtWords, kCtWords,
+                 ab, aa);
     __syncthreads();
   }
   uint64_t *outL = out + (static_cast<uint64_t>(b) * out_stride + 2ull * node) * kCtWords;
@@ -384,10 +405,8 @@ __device__ __forceinline__ void expand_body(const Dev4 &P, uint32_t galois_inv, 
     uint64_t vb[8], va[8];  // the key switch's delta in NTT form, canonical
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      vb[k] = opir60::fold<Q>(ab[k]);
-      vb[k] = min(vb[k], vb[k] - Q);
-      va[k] = opir60::fold<Q>(aa[k]);
-      va[k] = min(va[k], va[k] - Q);
+      vb[k] = min(ab[k], ab[k] - Q);
+      va[k] = min(aa[k], aa[k] - Q);
     }
     expand_tail_ntt<L>(P, galois, kshift, ct, vb, va, outL, outR);
     return;
@@ -395,13 +414,10 @@ __device__ __forceinline__ void expand_body(const Dev4 &P, uint32_t galois_inv, 
   {
     ulonglong2 wd[7];
     iload_d<L>(wd, P.T);
-    uint64_t vb[8], va[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { vb[k] = opir60::fold<Q>(ab[k]); va[k] = opir60::fold<Q>(aa[k]); }
-    iD<L>(vb, wd);
-    iD<L>(va, wd);
-    st_plane<3>(sm4, vb, tid);
-    st_plane<3>(sm4 + kPad, va, tid);
+    iD<L>(ab, wd);
+    iD<L>(aa, wd);
+    st_plane<3>(sm4, ab, tid);
+    st_plane<3>(sm4 + kPad, aa, tid);
   }
   __syncthreads();
   inv_mid<L>(sm4, 2, P.T);
@@ -460,9 +476,8 @@ k4_expand_level_ntt(Dev4 P, uint32_t galois, uint32_t galois_inv, uint32_t kshif
 // Expansion level, cluster split: with fewer nodes than SMs (the top of the
 // heap, and most levels of a single query) each node's key switch runs on a
 // cluster of C CTAs. CTA r NTTs digits [r D, (r + 1) D) (D = L_KS / C) of
-// sigma_k(c1) and accumulates their Shoup products with the key rows; the
-// partial sums (below 2q D each, their total below 16q as in the single-CTA
-// sum) meet in distributed shared memory; CTA 0 finishes the b part (c0 of
+// sigma_k(c1) and accumulates their products with the key rows; the folded
+// partial sums meet in distributed shared memory; CTA 0 finishes the b part (c0 of
 // both children), CTA 1 the a part (c1 of both children). Same children bit
 // for bit.
 template <int L, int C>
@@ -512,31 +527,7 @@ __device__ __forceinline__ void expand_split_body(const Dev4 &P, uint32_t galois
   }
   __syncthreads();
   fwd_mid<L>(sm4, D, P.T);
-  for (int e = 0; e < D; ++e) {
-    const int i = rank * D + e;
-    uint64_t v[8];
-    {
-      ulonglong2 wd[7];
-      fload_d<L>(wd, P.T);
-      ld_plane<3>(sm4 + e * kPad, v, tid);
-      fD<L>(v, wd);
-    }
-    const uint64_t *R = key + static_cast<uint64_t>(i) * kRowWords + L * kN + 8 * tid;
-    {
-      uint64_t w[8], ws[8];
-      ld8(R, w);
-      ld8(R + 4 * kN, ws);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) ab[k] += mul_shoup<Q>(v[k], w[k], ws[k]);
-    }
-    {
-      uint64_t w[8], ws[8];
-      ld8(R + 2 * kN, w);
-      ld8(R + 6 * kN, ws);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) aa[k] += mul_shoup<Q>(v[k], w[k], ws[k]);
-    }
-  }
+  mac_group<L>(P, sm4, D, key + static_cast<uint64_t>(rank) * D * kCtWords, kCtWords, ab, aa);
   __syncthreads();
   uint64_t *ex = sm4;  // [b / a][k][tid]
 #pragma unroll
@@ -614,14 +605,12 @@ k4_expand_level_split(Dev4 P, uint32_t galois_inv, uint32_t kshift,
 // decomposed ciphertext (both limbs read: y - x, or x when y is null) is
 // CRT-composed and split into l unsigned base-2^B digits; digit d of poly p
 // meets row p l + (l - 1 - d). Uses G planes (G = l when l <= 5, else 4).
-// Products are Shoup products in [0, 2q) with the rows' companions; the
-// sums are folded after each group (q + 16 c + 5 x 2q in between).
+// Sums are folded after each group.
 template <int L, int NL, int B>
 __device__ __forceinline__ void gadget_mac(const Dev4 &P, const uint64_t *x, const uint64_t *y,
                                            const uint64_t *rgsw, uint64_t *sm, uint64_t (&acc0)[8],
                                            uint64_t (&acc1)[8]) {
   constexpr int G = NL <= 5 ? NL : 4;
-  constexpr uint64_t Q = Limb<L>::q;
   const int tid = threadIdx.x;
 #pragma unroll 1
   for (int p = 0; p < 2; ++p) {
@@ -648,34 +637,8 @@ __device__ __forceinline__ void gadget_mac(const Dev4 &P, const uint64_t *x, con
       }
       __syncthreads();
       fwd_mid<L>(sm, G, P.T);
-      for (int e = 0; e < G; ++e) {
-        const int d = g * G + e;
-        const int row = p * NL + (NL - 1 - d);
-        uint64_t v[8];
-        {
-          ulonglong2 wd[7];
-          fload_d<L>(wd, P.T);
-          ld_plane<3>(sm + e * kPad, v, tid);
-          fD<L>(v, wd);
-        }
-        const uint64_t *R = rgsw + static_cast<uint64_t>(row) * kRowWords + L * kN + 8 * tid;
-        {
-          uint64_t w[8], ws[8];
-          ld8(R, w);
-          ld8(R + 4 * kN, ws);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) acc0[k] += mul_shoup<Q>(v[k], w[k], ws[k]);
-        }
-        {
-          uint64_t w[8], ws[8];
-          ld8(R + 2 * kN, w);
-          ld8(R + 6 * kN, ws);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) acc1[k] += mul_shoup<Q>(v[k], w[k], ws[k]);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < 8; ++k) { acc0[k] = opir60::fold<Q>(acc0[k]); acc1[k] = opir60::fold<Q>(acc1[k]); }
+      mac_group<L>(P, sm, G, rgsw + static_cast<uint64_t>(p * NL + NL - 1 - g * G) * kCtWords,
+                   -static_cast<int64_t>(kCtWords), acc0, acc1);
       __syncthreads();
     }
   }
@@ -691,21 +654,18 @@ __device__ __forceinline__ void selectors_body(const Dev4 &P, const Shape4 &S,
   const int row_id = blockIdx.x, b = blockIdx.z, tid = threadIdx.x;
   const int selno = row_id / S.l_ep, r = row_id % S.l_ep;
   const uint64_t *ct = leaves + (static_cast<uint64_t>(b) * leaf_stride + S.n0 + row_id) * kCtWords;
-  uint64_t *outs = sel + (static_cast<uint64_t>(b) * (S.num_dims - 1) + selno) * 2 * S.l_ep * kRowWords;
+  uint64_t *outs = sel + (static_cast<uint64_t>(b) * (S.num_dims - 1) + selno) * 2 * S.l_ep * kCtWords;
   uint64_t acc0[8], acc1[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) acc0[k] = acc1[k] = 0;
-  // bottom row: ExtProd(RGSW(s), row) with the key gadget; each selector row
-  // is stored with its Shoup companions (the MUX multiplies by it)
+  // bottom row: ExtProd(RGSW(s), row) with the key gadget
   gadget_mac<L, kLKey, kBaseKey>(P, ct, nullptr, gsw_keys[b], sm4, acc0, acc1);
-  uint64_t *bot = outs + static_cast<uint64_t>(S.l_ep + r) * kRowWords + L * kN + 8 * tid;
+  uint64_t *bot = outs + static_cast<uint64_t>(S.l_ep + r) * kCtWords + L * kN + 8 * tid;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const uint64_t v0 = min(acc0[k], acc0[k] - Q), v1 = min(acc1[k], acc1[k] - Q);
     bot[k] = v0;
     bot[2 * kN + k] = v1;
-    bot[4 * kN + k] = shoup_of<Q>(v0);
-    bot[6 * kN + k] = shoup_of<Q>(v1);
   }
   // top row: the expanded row itself in NTT form (gsw.cpp:330-338)
 #pragma unroll
@@ -720,7 +680,7 @@ __device__ __forceinline__ void selectors_body(const Dev4 &P, const Shape4 &S,
   fwd_mid<L>(sm4, 2, P.T);
   ulonglong2 wd[7];
   fload_d<L>(wd, P.T);
-  uint64_t *top = outs + static_cast<uint64_t>(r) * kRowWords + L * kN + 8 * tid;
+  uint64_t *top = outs + static_cast<uint64_t>(r) * kCtWords + L * kN + 8 * tid;
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
     uint64_t v[8];
@@ -728,9 +688,7 @@ __device__ __forceinline__ void selectors_body(const Dev4 &P, const Shape4 &S,
     fD<L>(v, wd);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const uint64_t c = opir60::canon<Q>(v[k]);
-      top[p * 2 * kN + k] = c;
-      top[4 * kN + p * 2 * kN + k] = shoup_of<Q>(c);
+      top[p * 2 * kN + k] = opir60::canon<Q>(v[k]);
     }
   }
 }
@@ -940,7 +898,7 @@ __device__ __forceinline__ void mux_body(const Dev4 &P, const Shape4 &S, uint32_
   else { xi = i; yi = i + half; oi = i; }
   const uint64_t *x = base_in + static_cast<uint64_t>(xi) * kCtWords;
   const uint64_t *y = base_in + static_cast<uint64_t>(yi) * kCtWords;
-  const uint64_t *rgsw = sel + (static_cast<uint64_t>(b) * (S.num_dims - 1) + level) * 2 * kLEp * kRowWords;
+  const uint64_t *rgsw = sel + (static_cast<uint64_t>(b) * (S.num_dims - 1) + level) * 2 * kLEp * kCtWords;
   uint64_t acc0[8], acc1[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) acc0[k] = acc1[k] = 0;
@@ -985,16 +943,14 @@ k4_mux_level(Dev4 P, Shape4 S, uint32_t level, uint32_t n_pairs, uint32_t offset
 // MUX level, cluster split: with fewer pairs than SMs each MUX runs on a
 // cluster of C CTAs. CTA r takes digits [d0, d0 + dn) of polynomial p of
 // y - x (C = 2: p = r, all l digits; C = 4: p = r / 2, digits 0-2 or 3-4),
-// accumulates their Shoup products with the RGSW rows and folds them; CTAs 0
-// and 1 add the partials through distributed shared memory, fold them and
-// finish output polynomial c0 / c1 (INTT,
-// + x). The same residues enter the same INTT: bit for bit the single-CTA
-// MUX.
+// accumulates their products with the RGSW rows, folded; CTAs 0 and 1 add
+// the partials through distributed shared memory, fold them and finish output
+// polynomial c0 / c1 (INTT, + x). The same residues enter the same INTT: bit
+// for bit the single-CTA MUX.
 template <int L>
 __device__ __forceinline__ void gadget_part(const Dev4 &P, const uint64_t *x, const uint64_t *y,
                                             const uint64_t *rgsw, uint64_t *sm, int p, int d0,
                                             int dn, uint64_t (&acc0)[8], uint64_t (&acc1)[8]) {
-  constexpr uint64_t Q = Limb<L>::q;
   const int tid = threadIdx.x;
   {
     u128 u[8];
@@ -1015,33 +971,8 @@ __device__ __forceinline__ void gadget_part(const Dev4 &P, const uint64_t *x, co
   }
   __syncthreads();
   fwd_mid<L>(sm, dn, P.T);
-  for (int e = 0; e < dn; ++e) {
-    const int row = p * kLEp + (kLEp - 1 - (d0 + e));
-    uint64_t v[8];
-    {
-      ulonglong2 wd[7];
-      fload_d<L>(wd, P.T);
-      ld_plane<3>(sm + e * kPad, v, tid);
-      fD<L>(v, wd);
-    }
-    const uint64_t *R = rgsw + static_cast<uint64_t>(row) * kRowWords + L * kN + 8 * tid;
-    {
-      uint64_t w[8], ws[8];
-      ld8(R, w);
-      ld8(R + 4 * kN, ws);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc0[k] += mul_shoup<Q>(v[k], w[k], ws[k]);
-    }
-    {
-      uint64_t w[8], ws[8];
-      ld8(R + 2 * kN, w);
-      ld8(R + 6 * kN, ws);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc1[k] += mul_shoup<Q>(v[k], w[k], ws[k]);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) { acc0[k] = opir60::fold<Q>(acc0[k]); acc1[k] = opir60::fold<Q>(acc1[k]); }
+  mac_group<L>(P, sm, dn, rgsw + static_cast<uint64_t>(p * kLEp + kLEp - 1 - d0) * kCtWords,
+               -static_cast<int64_t>(kCtWords), acc0, acc1);
   __syncthreads();
 }
 
@@ -1064,7 +995,7 @@ __device__ __forceinline__ void mux_split_body(const Dev4 &P, const Shape4 &S, u
   const uint64_t *base_in = in + static_cast<uint64_t>(b) * mid_stride * kCtWords;
   const uint64_t *x = base_in + static_cast<uint64_t>(i) * xs * kCtWords;
   const uint64_t *y = base_in + (static_cast<uint64_t>(i) * xs + yoff) * kCtWords;
-  const uint64_t *rgsw = sel + (static_cast<uint64_t>(b) * (S.num_dims - 1) + level) * 2 * kLEp * kRowWords;
+  const uint64_t *rgsw = sel + (static_cast<uint64_t>(b) * (S.num_dims - 1) + level) * 2 * kLEp * kCtWords;
   uint64_t acc0[8], acc1[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) acc0[k] = acc1[k] = 0;

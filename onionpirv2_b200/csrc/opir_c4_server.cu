@@ -27,17 +27,6 @@ namespace {
 
 constexpr uint32_t kLKsRows = 8, kLKeyRows = 8;  // L_KS, L_KEY of both sets
 
-// Appends one ciphertext-shaped row (2 N limbs u64, limb-major polynomials)
-// and its Shoup companions floor(w 2^64 / q_limb) in the device row layout.
-void append_row(std::vector<uint64_t> &dst, const uint64_t *row, uint32_t n, uint32_t limbs) {
-  const uint64_t ct = 2ull * n * limbs;
-  dst.insert(dst.end(), row, row + ct);
-  for (uint64_t j = 0; j < ct; ++j) {
-    const uint64_t q = (limbs == 2 && ((j / n) & 1)) ? kQ1 : kQ0;
-    dst.push_back(static_cast<uint64_t>((static_cast<unsigned __int128>(row[j]) << 64) / q));
-  }
-}
-
 uint32_t resp_bytes_of(const opir_params &p) {
   return static_cast<uint32_t>((2ull * p.poly_degree * p.small_q_width + 7) / 8);
 }
@@ -70,12 +59,12 @@ struct Plan {
   uint64_t bytes() const { return (2 * lvl + sel + 2 * mid + resp) * 8 + keyptrs * sizeof(void *); }
 };
 
-// ct: u64 words per ciphertext (2 N limbs); row = 2 ct (with companions)
+// ct: u64 words per ciphertext (2 N limbs)
 Plan plan_for(const Shape4 &s, uint64_t lvl_slots, uint32_t n, uint32_t N, uint64_t ct) {
   const uint64_t nsel = s.num_dims > 1 ? s.num_dims - 1 : 0;
   Plan pl{};
   pl.lvl = static_cast<size_t>(n) * lvl_slots * ct;
-  pl.sel = std::max<uint64_t>(1, n * nsel * 2 * s.l_ep * 2 * ct);
+  pl.sel = std::max<uint64_t>(1, n * nsel * 2 * s.l_ep * ct);
   pl.mid = static_cast<size_t>(n) * s.other * ct;
   pl.resp = static_cast<size_t>(n) * 2 * N;
   pl.keyptrs = 2ull * n;
@@ -94,7 +83,6 @@ Server::Server(const opir_params &p, cudaStream_t stream, const opir::RowShard *
   n_ = p_.poly_degree;
   limbs_ = p_.num_limbs;
   ct_ = 2ull * n_ * limbs_;
-  row_ = 2 * ct_;
   out_words_ = 2ull * n_;
   sh_ = shape_of(p_);
   tree_h_ = sh_.num_dims > 1 ? sh_.num_dims - 1 : 0;
@@ -342,21 +330,13 @@ void Server::set_client_keys(uint64_t id, const uint64_t *bv_keys, const uint32_
   }
   const size_t gsw_rows = 2ull * kLKeyRows;
   check_ct_values(gsw_key, gsw_rows);
-  // device rows carry their Shoup companions (opir_c4_kernels.h)
-  std::vector<uint64_t> bv_rows, gsw_rows_host;
-  bv_rows.reserve(static_cast<size_t>(h) * kLKsRows * row_);
-  for (uint32_t d = 0; d < h; ++d)
-    for (uint32_t r = 0; r < kLKsRows; ++r)
-      append_row(bv_rows, bv_keys + order[d] * key_words + r * ct_, n_, limbs_);
-  for (size_t r = 0; r < gsw_rows; ++r) append_row(gsw_rows_host, gsw_key + r * ct_, n_, limbs_);
   Keys k;
-  k.bv.alloc(std::max<size_t>(1, bv_rows.size()));
-  k.gsw.alloc(gsw_rows_host.size());
-  if (!bv_rows.empty())
-    ck(cudaMemcpyAsync(k.bv.p, bv_rows.data(), bv_rows.size() * 8, cudaMemcpyHostToDevice, st_),
-       "bv upload");
-  ck(cudaMemcpyAsync(k.gsw.p, gsw_rows_host.data(), gsw_rows_host.size() * 8,
-                     cudaMemcpyHostToDevice, st_), "gsw upload");
+  k.bv.alloc(std::max<size_t>(1, static_cast<size_t>(h) * key_words));
+  k.gsw.alloc(gsw_rows * ct_);
+  for (uint32_t d = 0; d < h; ++d)
+    ck(cudaMemcpyAsync(k.bv.p + d * key_words, bv_keys + order[d] * key_words, key_words * 8,
+                       cudaMemcpyHostToDevice, st_), "bv upload");
+  ck(cudaMemcpyAsync(k.gsw.p, gsw_key, gsw_rows * ct_ * 8, cudaMemcpyHostToDevice, st_), "gsw upload");
   ck(cudaStreamSynchronize(st_), "key upload");
   Keys &slot = clients_[id];
   slot.bv.swap(k.bv);
@@ -455,7 +435,7 @@ void Server::stage_in(const uint64_t *d_queries, uint32_t n) {
 // OPIR_NTT_LEAVES=0 turns it off), the last level writes the first n0
 // leaves in NTT form and *ntt_first is set.
 const uint64_t *Server::run_expand(uint32_t n, bool *ntt_first) {
-  const uint64_t level_stride = static_cast<uint64_t>(kLKsRows) * row_;
+  const uint64_t level_stride = static_cast<uint64_t>(kLKsRows) * ct_;
   const char *env = std::getenv("OPIR_NTT_LEAVES");
   // a single query keeps the coefficient path: its last level is too
   // small for the NTT-form tail to pay for itself (CONFIG_N2048_K1 batch 1:
@@ -731,10 +711,8 @@ void Server::complete_selectors(uint64_t id, const uint64_t *expanded, uint64_t 
   ck(cudaMemcpyAsync(lvl_[0].p, expanded, static_cast<size_t>(sh_.useful) * ct_ * 8,
                      cudaMemcpyHostToDevice, st_), "upload");
   run_selectors(lvl_[0].p, keyptrs_.p + 1, 1);
-  // the rows without their Shoup companions
-  ck(cudaMemcpy2DAsync(out, ct_ * 8, sel_.p, row_ * 8, ct_ * 8,
-                       static_cast<size_t>(nsel) * 2 * sh_.l_ep, cudaMemcpyDeviceToHost, st_),
-     "download");
+  ck(cudaMemcpyAsync(out, sel_.p, static_cast<size_t>(nsel) * 2 * sh_.l_ep * ct_ * 8,
+                     cudaMemcpyDeviceToHost, st_), "download");
   ck(cudaStreamSynchronize(st_), "complete_selectors");
 }
 
@@ -760,14 +738,9 @@ void Server::evaluate_other_dim(const uint64_t *mid, const uint64_t *selectors, 
   ensure_capacity(1);
   ck(cudaMemcpyAsync(mid_[0].p, mid, static_cast<size_t>(sh_.other) * ct_ * 8,
                      cudaMemcpyHostToDevice, st_), "upload");
-  std::vector<uint64_t> rows;
-  if (nsel) {
-    const size_t n_rows = static_cast<size_t>(nsel) * 2 * sh_.l_ep;
-    rows.reserve(n_rows * row_);
-    for (size_t r = 0; r < n_rows; ++r) append_row(rows, selectors + r * ct_, n_, limbs_);
-    ck(cudaMemcpyAsync(sel_.p, rows.data(), rows.size() * 8, cudaMemcpyHostToDevice, st_),
-       "upload");
-  }
+  if (nsel)
+    ck(cudaMemcpyAsync(sel_.p, selectors, static_cast<size_t>(nsel) * 2 * sh_.l_ep * ct_ * 8,
+                       cudaMemcpyHostToDevice, st_), "upload");
   const uint64_t *r = run_other_dims(1);
   ck(cudaMemcpyAsync(out, r, ct_ * 8, cudaMemcpyDeviceToHost, st_), "download");
   ck(cudaStreamSynchronize(st_), "evaluate_other_dim");
@@ -782,16 +755,13 @@ void Server::ext_prod_mux(const uint64_t *x, const uint64_t *y, const uint64_t *
   Shape4 sh = sh_;  // one MUX level of a two-candidate tree
   sh.other = 2;
   sh.num_dims = 2;
-  std::vector<uint64_t> rows;
-  rows.reserve(n_rows * row_);
-  for (size_t r = 0; r < n_rows; ++r) append_row(rows, sel + r * ct_, n_, limbs_);
   opir::DevBuf<uint64_t> xy, res, srows;
   xy.alloc(2 * ct_);
   res.alloc(2 * ct_);
-  srows.alloc(rows.size());
+  srows.alloc(n_rows * ct_);
   ck(cudaMemcpyAsync(xy.p, x, ct_ * 8, cudaMemcpyHostToDevice, st_), "upload");
   ck(cudaMemcpyAsync(xy.p + ct_, y, ct_ * 8, cudaMemcpyHostToDevice, st_), "upload");
-  ck(cudaMemcpyAsync(srows.p, rows.data(), rows.size() * 8, cudaMemcpyHostToDevice, st_), "upload");
+  ck(cudaMemcpyAsync(srows.p, sel, n_rows * ct_ * 8, cudaMemcpyHostToDevice, st_), "upload");
   run_mux(sh, 0, 1, xy.p, res.p, 2, srows.p, 1);
   ck(cudaMemcpyAsync(out, res.p, ct_ * 8, cudaMemcpyDeviceToHost, st_), "download");
   ck(cudaStreamSynchronize(st_), "ext_prod_mux");
@@ -813,7 +783,7 @@ void Server::tree_select_device(const uint64_t *d_leaves, const uint64_t *d_sele
                      cudaMemcpyDeviceToDevice, st_), "alpha copy");
   run_first_dim(lvl_[0].p, 1, nullptr);
   const uint32_t fold = static_cast<uint32_t>(fold_count);
-  const size_t sel_words = 2ull * sh_.l_ep * row_;  // one selector with companions
+  const size_t sel_words = 2ull * sh_.l_ep * ct_;  // one selector
   for (uint32_t a = 1; a <= fold; ++a) {  // MSB-first: step a takes selector begin+count-a
     const uint64_t u = fold_begin + fold_count - a;
     ck(cudaMemcpyAsync(sel_.p + a * sel_words, d_selectors + u * sel_words, sel_words * 8,
@@ -834,14 +804,11 @@ void Server::select_fold(const uint64_t *alpha, const uint64_t *fold_sel, uint32
                      cudaMemcpyHostToDevice, st_), "upload");
   run_first_dim(lvl_[0].p, 1, nullptr);
   const uint64_t *res = mid_[0].p;
-  std::vector<uint64_t> rows;
   if (fold) {
-    const size_t n_rows = static_cast<size_t>(fold) * 2 * sh_.l_ep;
-    rows.reserve(n_rows * row_);
-    for (size_t r = 0; r < n_rows; ++r) append_row(rows, fold_sel + r * ct_, n_, limbs_);
+    const size_t sel_words = 2ull * sh_.l_ep * ct_;
     // slot 0 of the selector set is unused: step a takes slot a
-    ck(cudaMemcpyAsync(sel_.p + 2ull * sh_.l_ep * row_, rows.data(), rows.size() * 8,
-                       cudaMemcpyHostToDevice, st_), "upload");
+    ck(cudaMemcpyAsync(sel_.p + sel_words, fold_sel, fold * sel_words * 8, cudaMemcpyHostToDevice, st_),
+       "upload");
     for (uint32_t a = 1; a <= fold; ++a)
       run_mux(sh_, a, sh_.num_dims - 1, mid_[(a - 1) & 1].p, mid_[a & 1].p, sh_.other, sel_.p, 1);
     res = mid_[fold & 1].p;

@@ -93,7 +93,7 @@ class Server {
   // Device-resident tree (opir_tree_query), on the handle's stream, after
   // reserve(1). Query-shape handle: unpack_tree_query of a host query into
   // the handle's leaves (tree_leaves(), n0 alpha ciphertexts first) and
-  // selector rows (tree_selectors(), 2 L_EP rows of kRowWords per selector).
+  // selector rows (tree_selectors(), 2 L_EP ciphertexts per selector).
   void tree_unpack(uint64_t id, const uint64_t *query);
   const uint64_t *tree_leaves() const { return lvl_[sh_.h & 1].p; }
   const uint64_t *tree_selectors() const { return sel_.p; }
@@ -148,7 +148,6 @@ class Server {
   uint32_t n_ = kN;          // ring degree N
   uint32_t limbs_ = 2;       // RNS limbs K
   uint64_t ct_ = kCtWords;   // u64 words per ciphertext: 2 N K
-  uint64_t row_ = kRowWords; // u64 words per key / selector row: ciphertext + companions
   Shape4 sh_{};
   Dev4 dp_{};
   cudaStream_t st_ = nullptr;

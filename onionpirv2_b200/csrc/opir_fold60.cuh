@@ -86,6 +86,39 @@ __device__ __forceinline__ uint64_t mul(uint64_t a, ulonglong2 w) {
   return join<Q>(A0, A1);
 }
 
+// Key products, summed without reduction: with v = v0 + 2^30 v1 and a row word
+// w = w0 + 2^30 w1 < q,
+//   lo += v0 w0,   hi += v1 w1,   mix += (v0 + v1)(w0 + w1)
+// (Karatsuba; mix only counts mod 2^64) take up to five products and a folded
+// sum: lo, hi < 5 2^60 + 2^61, mix - lo - hi < 5 2^61. Three multiply-adds a
+// product and one join per sum, against Shoup's high and two low 64-bit
+// products and a second stored word per row word.
+// v folded, in limbs v0 | v1 << 32 (v1 <= 2^30)
+template <uint64_t Q>
+__device__ __forceinline__ uint64_t limbs(uint64_t v) {
+  const uint64_t x = fold<Q>(v);
+  return (x & kLow30) | ((x >> 30) << 32);
+}
+__device__ __forceinline__ void mac(uint64_t &lo, uint64_t &hi, uint64_t &mix, uint64_t v, uint64_t w) {
+  const uint32_t v0 = static_cast<uint32_t>(v), v1 = static_cast<uint32_t>(v >> 32);
+  const uint32_t w0 = static_cast<uint32_t>(w) & kLow30, w1 = static_cast<uint32_t>(w >> 30);
+  lo = mad32(v0, w0, lo);
+  hi = mad32(v1, w1, hi);
+  mix = mad32(v0 + v1, w0 + w1, mix);
+}
+// lo + 2^30 (mix - lo - hi) + 2^60 hi (mod q), below q + 16 c: 2^60 hi = c hi
+// with c hi = c (hi mod 2^32) + 2^32 y, y = c (hi >> 32) < 2^49, and 2^32 y =
+// c (y >> 28) + 2^32 (y mod 2^28). Sum for join(): below 5 2^60 + 2^61 + 2^50.
+template <uint64_t Q>
+__device__ __forceinline__ uint64_t mac_join(uint64_t lo, uint64_t hi, uint64_t mix) {
+  constexpr uint32_t c = Fold<Q>::c;
+  const uint64_t y = mul32(static_cast<uint32_t>(hi >> 32), c);
+  uint64_t r = mad32(static_cast<uint32_t>(hi), c, lo);
+  r = mad32(static_cast<uint32_t>(y >> 28), c, r);
+  r += (y & 0xFFFFFFFull) << 32;
+  return join<Q>(r, mix - lo - hi);
+}
+
 // Forward butterfly (x, y) -> (x + w y, x - w y + q). With inputs in
 // [q, 2q) (First adds that q to canonical ones) twelve stages stay between
 // q - 12 16 c > 0 and 14 q + 192 c < 2^64.

@@ -8,8 +8,7 @@
 // about q a stage and stay below 2^64, inverse passes begin and end folded.
 // Merged Cooley-Tukey forward with bit-reversed output, Gentleman-Sande
 // inverse scaled by N^-1 (the HEXL convention the reference registers,
-// utils.cpp:26-56). Key and selector rows carry Shoup companions, so every
-// key product is three 64-bit multiplies landing in [0, 2q).
+// utils.cpp:26-56).
 #include "opir_k1p_kernels.h"
 
 #include "opir_fold60.cuh"
@@ -85,10 +84,6 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {  // splitmix64 finaliser
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
   return z ^ (z >> 31);
 }
-// a w mod q in [0, 2q) for any 64-bit a (Shoup)
-__device__ __forceinline__ uint64_t mulsh(uint64_t a, uint64_t w, uint64_t ws) {
-  return a * w - __umul64hi(a, ws) * kQ;
-}
 __device__ __forceinline__ uint64_t fold2(uint64_t x) { return min(x, x - kQ); }  // [0, 2q)
 __device__ __forceinline__ uint64_t add_q(uint64_t a, uint64_t b) {
   const uint64_t s = a + b;
@@ -99,9 +94,6 @@ __device__ __forceinline__ uint64_t sub_q(uint64_t a, uint64_t b) {
   return min(d, d - kQ);
 }
 __device__ __forceinline__ uint64_t neg_q(uint64_t a) { return a ? kQ - a : 0; }
-__device__ __forceinline__ uint64_t shoup_of(uint64_t w) {
-  return static_cast<uint64_t>((static_cast<u128>(w) << 64) / kQ);
-}
 // Balanced base-2^B digits, LSB first (gsw.cpp:277-293, bv_keyswitch.cpp:
 // 20-40): v in [0, q) is centred to c in (-q/2, q/2]; c + C with
 // C = 2^(B-1) sum_{i<L} 2^(B i) has plain base-2^B digits u_i = r_i + 2^(B-1)
@@ -275,20 +267,53 @@ __device__ __forceinline__ void ld4(const uint64_t *p, uint64_t *v) {
   const ulonglong2 b = __ldg(reinterpret_cast<const ulonglong2 *>(p + 2));
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
-// acc_k += v_k * row polynomial `part` (of a row [p0][p1][p0'][p1'], each N),
-// each product in [0, 2q)
-__device__ __forceinline__ void mac_part(const uint64_t *row, int part, const uint64_t (&v)[8],
-                                         uint64_t (&acc)[8], int tid) {
+// acc0 / acc1 += sum over np <= 5 planes of NTT(plane e) x row e's polynomial
+// 0 / 1: pass D of the planes, then the products with rows [p0][p1], `stride`
+// words apart; folded on entry and exit. The two halves of a thread's
+// coefficients go one after the other, so 24 64-bit sums are live, not 48.
+// Batch 32 of 2^18 entries: 10.13 ms, with Shoup products 10.48.
+__device__ __forceinline__ void mac_group(const Dev1 &P, const uint64_t *sm, int np,
+                                          const uint64_t *row, int64_t stride,
+                                          uint64_t (&acc0)[8], uint64_t (&acc1)[8], int tid) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    const int j0 = 4 * (tid + 256 * h);
-    uint64_t w[4], ws[4];
-    ld4(row + part * kN + j0, w);
-    ld4(row + (2 + part) * kN + j0, ws);
+    const int b4 = tid + 256 * h, j0 = 4 * b4;
+    const ulonglong2 w0 = __ldg(P.fwt + 512 + b4), w1 = __ldg(P.fwt + 1024 + 2 * b4),
+                     w2 = __ldg(P.fwt + 1025 + 2 * b4);
+    uint64_t hi0[4], mix0[4], hi1[4], mix1[4];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) acc[4 * h + m] += mulsh(v[4 * h + m], w[m], ws[m]);
+    for (int m = 0; m < 4; ++m) {
+      hi0[m] = hi1[m] = 0;
+      mix0[m] = acc0[4 * h + m];
+      mix1[m] = acc1[4 * h + m];
+    }
+    const uint64_t *R = row + j0;
+#pragma unroll 1
+    for (int e = 0; e < np; ++e, R += stride) {
+      uint64_t u[4], a[4], b[4];
+      ld4(R, a);
+      ld4(R + kN, b);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) u[m] = sm[e * kPad + padi(j0 + m)];
+      opir60::fbf<kQ>(u[0], u[2], w0);
+      opir60::fbf<kQ>(u[1], u[3], w0);
+      opir60::fbf<kQ>(u[0], u[1], w1);
+      opir60::fbf<kQ>(u[2], u[3], w2);
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const uint64_t v = opir60::limbs<kQ>(u[m]);
+        opir60::mac(acc0[4 * h + m], hi0[m], mix0[m], v, a[m]);
+        opir60::mac(acc1[4 * h + m], hi1[m], mix1[m], v, b[m]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      acc0[4 * h + m] = opir60::mac_join<kQ>(acc0[4 * h + m], hi0[m], mix0[m]);
+      acc1[4 * h + m] = opir60::mac_join<kQ>(acc1[4 * h + m], hi1[m], mix1[m]);
+    }
   }
 }
+
 // ------------------------------------------------------------ DB preprocessing
 // server.cpp:80-203 with one prime: pt mod q, NTT, the coefficient-major
 // transpose as eight byte planes per NTT level, db8[(z 8 + plane)][row][n0p].
@@ -362,7 +387,7 @@ k1p_db_preprocess(Dev1 P, const uint64_t *__restrict__ coeffs, uint64_t coeff_pt
 // One heap node per CTA: the BV key switch (bv_keyswitch.cpp:296-367) of the
 // node and its two children (server.cpp:794-809): left = c + c', right =
 // (c - c') X^-k, sigma_k(c)[j] = +-c[j k^-1 mod 2N]. Digits in groups of 4
-// planes; sums of Shoup key products folded after each group.
+// planes, sums folded after each group.
 constexpr int kGroup = 4;
 
 // Children of the last level in NTT form (the first-dimension leaves), from
@@ -444,7 +469,7 @@ __device__ __forceinline__ void expand_body(const Dev1 &P, uint32_t galois_inv, 
   extern __shared__ uint64_t sm1[];
   const int node = node0 + blockIdx.x, b = blockIdx.z, tid = threadIdx.x;
   const uint64_t *ct = in + (static_cast<uint64_t>(b) * in_stride + node) * kCtWords;
-  const uint64_t *key = bv_keys[b] + bv_level_off;  // rows [b][a][b'][a']
+  const uint64_t *key = bv_keys[b] + bv_level_off;  // rows [b][a]
   uint64_t u[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
@@ -467,18 +492,7 @@ __device__ __forceinline__ void expand_body(const Dev1 &P, uint32_t galois_inv, 
     }
     __syncthreads();
     fwd_mid(sm1, kGroup, P.fwt);
-    ulonglong2 wd[6];
-    load_d(wd, P.fwt, tid);
-    for (int e = 0; e < kGroup; ++e) {
-      const uint64_t *R = key + static_cast<uint64_t>(g * kGroup + e) * kRowWords;
-      uint64_t v[8];
-      ld_plane<3>(sm1 + e * kPad, v, tid);
-      fD(v, wd);
-      mac_part(R, 0, v, ab, tid);
-      mac_part(R, 1, v, aa, tid);
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { ab[k] = opir60::fold<kQ>(ab[k]); aa[k] = opir60::fold<kQ>(aa[k]); }
+    mac_group(P, sm1, kGroup, key + static_cast<uint64_t>(g) * kGroup * kCtWords, kCtWords, ab, aa, tid);
     __syncthreads();
   }
   uint64_t *outL = out + (static_cast<uint64_t>(b) * out_stride + 2ull * node) * kCtWords;
@@ -585,19 +599,9 @@ __device__ __forceinline__ void gadget_mac(const Dev1 &P, const uint64_t *x, con
       }
       __syncthreads();
       fwd_mid<Full>(sm, G, P.fwt);
-      ulonglong2 wd[6];
-      load_d(wd, P.fwt, tid);
-      for (int e = 0; e < G; ++e) {
-        const int d = g * G + e;
-        const uint64_t *R = rgsw + static_cast<uint64_t>(p * L + (L - 1 - d)) * kRowWords;
-        uint64_t v[8];
-        ld_plane<3>(sm + e * kPad, v, tid);
-        fD(v, wd);
-        mac_part(R, 0, v, acc0, tid);  // row [c0][c1][c0'][c1']
-        mac_part(R, 1, v, acc1, tid);
-      }
-#pragma unroll
-      for (int k = 0; k < 8; ++k) { acc0[k] = opir60::fold<kQ>(acc0[k]); acc1[k] = opir60::fold<kQ>(acc1[k]); }
+      // digit d meets row p L + (L - 1 - d)
+      mac_group(P, sm, G, rgsw + static_cast<uint64_t>(p * L + L - 1 - g * G) * kCtWords,
+                -static_cast<int64_t>(kCtWords), acc0, acc1, tid);
       __syncthreads();
     }
   }
@@ -606,7 +610,7 @@ __device__ __forceinline__ void gadget_mac(const Dev1 &P, const uint64_t *x, con
 // ------------------------------------------------------------ selectors
 // complete_selectors / query_to_gsw (server.cpp:823-855, gsw.cpp:317-357):
 // the top row is the expanded row itself in NTT form, the bottom row its
-// external product with RGSW(s); both stored with Shoup companions.
+// external product with RGSW(s).
 template <int MINB>
 __global__ void __launch_bounds__(kThreads, MINB)
 k1p_selectors(Dev1 P, Shape1 S, const uint64_t *__restrict__ leaves, uint64_t leaf_stride,
@@ -615,20 +619,18 @@ k1p_selectors(Dev1 P, Shape1 S, const uint64_t *__restrict__ leaves, uint64_t le
   const int row_id = blockIdx.x, b = blockIdx.z, tid = threadIdx.x;
   const int selno = row_id / S.l_ep, r = row_id % S.l_ep;
   const uint64_t *ct = leaves + (static_cast<uint64_t>(b) * leaf_stride + S.n0 + row_id) * kCtWords;
-  uint64_t *outs = sel + (static_cast<uint64_t>(b) * (S.num_dims - 1) + selno) * 2 * S.l_ep * kRowWords;
+  uint64_t *outs = sel + (static_cast<uint64_t>(b) * (S.num_dims - 1) + selno) * 2 * S.l_ep * kCtWords;
   uint64_t acc0[8], acc1[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) acc0[k] = acc1[k] = 0;
   gadget_mac<kLKey, kBaseKey, false>(P, ct, nullptr, gsw_keys[b], sm1, acc0, acc1);
-  uint64_t *bot = outs + static_cast<uint64_t>(S.l_ep + r) * kRowWords;
+  uint64_t *bot = outs + static_cast<uint64_t>(S.l_ep + r) * kCtWords;
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const int j = posD(tid, k);
     const uint64_t v0 = fold2(acc0[k]), v1 = fold2(acc1[k]);
     bot[j] = v0;
     bot[kN + j] = v1;
-    bot[2 * kN + j] = shoup_of(v0);
-    bot[3 * kN + j] = shoup_of(v1);
   }
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
@@ -642,7 +644,7 @@ k1p_selectors(Dev1 P, Shape1 S, const uint64_t *__restrict__ leaves, uint64_t le
   fwd_mid<false>(sm1, 2, P.fwt);
   ulonglong2 wd[6];
   load_d(wd, P.fwt, tid);
-  uint64_t *top = outs + static_cast<uint64_t>(r) * kRowWords;
+  uint64_t *top = outs + static_cast<uint64_t>(r) * kCtWords;
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
     uint64_t v[8];
@@ -651,9 +653,7 @@ k1p_selectors(Dev1 P, Shape1 S, const uint64_t *__restrict__ leaves, uint64_t le
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int j = posD(tid, k);
-      const uint64_t c = opir60::canon<kQ>(v[k]);
-      top[p * kN + j] = c;
-      top[2 * kN + p * kN + j] = shoup_of(c);
+      top[p * kN + j] = opir60::canon<kQ>(v[k]);
     }
   }
 }
@@ -816,7 +816,7 @@ k1p_mux_level(Dev1 P, Shape1 S, uint32_t level, uint32_t n_pairs, uint32_t offse
   const uint64_t *x = base_in + static_cast<uint64_t>(xi) * kCtWords;
   const uint64_t *y = base_in + static_cast<uint64_t>(yi) * kCtWords;
   const uint64_t *rgsw =
-      sel + (static_cast<uint64_t>(b) * (S.num_dims - 1) + level) * 2 * kLEp * kRowWords;
+      sel + (static_cast<uint64_t>(b) * (S.num_dims - 1) + level) * 2 * kLEp * kCtWords;
   uint64_t acc0[8], acc1[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) acc0[k] = acc1[k] = 0;

@@ -12,11 +12,9 @@
 //                `plane` of the reference's db[level * num_pt + pt],
 //                pt = row n0 + col (server.cpp:172-194), rows padded to
 //                n0p = n0 rounded up to 16
-//   BV keys    : per client [level < h][row < L_KS][b (N)][a (N)][b' (N)]
-//                [a' (N)], NTT form, w' = floor(w 2^64 / q) the Shoup
-//                companion of w (kRowWords per row)
-//   RGSW key   : per client [row < 2 L_KEY][c0][c1][c0'][c1'], NTT form
-//   selectors  : [query][dim < num_dims-1][row < 2 L_EP][c0][c1][c0'][c1']
+//   BV keys    : per client [level < h][row < L_KS][b (N)][a (N)], NTT form
+//   RGSW key   : per client [row < 2 L_KEY][c0][c1], NTT form
+//   selectors  : [query][dim < num_dims-1][row < 2 L_EP][c0][c1], NTT form
 //   query mat  : qm[col < 2 B][k < n0][z < N] u64, col = 2 query + poly, then
 //                qb[(z 8 + plane)][col][n0p] bytes
 //   cmat       : [z][col][row] u64 (the 64-bit-limb scan's output layout)
@@ -36,7 +34,6 @@ namespace opir1 {
 constexpr int kN = 2048;
 constexpr uint64_t kQ = 1152921504606830593ull;  // 2^60 - 2^14 + 1
 constexpr int kCtWords = 2 * kN;   // u64 words per ciphertext
-constexpr int kRowWords = 4 * kN;  // a key / RGSW row: ciphertext + Shoup companions
 constexpr int kLEp = 5, kBaseEp = 12, kLKey = 8, kBaseKey = 8, kLKs = 8, kBaseKs = 8;
 
 struct Dev1 {
