@@ -16,9 +16,8 @@
 // columns [i ntile, (i + 8) ntile): the accumulator of S_s is columns
 // [s ntile, (s + 1) ntile). The first K step of a tile initialises each
 // column once: A_0 Q_0..7 (overwrite S_0..7), A_7 Q_1..7 (overwrite S_8..14),
-// then A_7 Q_0 and A_1..6 Q_0..7 accumulate. The epilogue forms
-// lo = sum_{s<8} S_s 2^(8s) and hi = sum_{s>=8} S_s 2^(8(s-8)) exactly and
-// returns (lo + (hi mod q) (2^64 mod q)) mod q.
+// then A_7 Q_0 and A_1..6 Q_0..7 accumulate. The epilogue forms the classes'
+// sum in four words of 56 bits and folds them modulo q = 2^60 - c.
 //
 // Structure (as the single-modulus tensor-core scan): persistent CTAs, 10
 // warps -- TMA producer, TMEM owner + MMA issuer, 8 epilogue warps (two per
@@ -43,6 +42,7 @@
 #include <string>
 
 #include "opir_c4_kernels.h"
+#include "opir_fold60.cuh"
 #include "opir_tc.cuh"
 
 namespace opir4 {
@@ -50,7 +50,6 @@ namespace opir4 {
 namespace {
 
 using namespace opir::tc;
-using u128 = unsigned __int128;
 
 constexpr int kM = 128;
 constexpr int kKT = 64;             // K bytes per stage (64-byte swizzle)
@@ -64,26 +63,27 @@ constexpr uint32_t kTmemCols = 512;
 constexpr size_t kSmemLimit = 227 * 1024;
 constexpr long long kPairWaitCycles = 40000;  // ~20 us
 
-template <uint64_t Q>
-__device__ __forceinline__ uint64_t red128_tc(u128 x) {  // x < 2^126 -> [0, q)
-  constexpr uint64_t c = static_cast<uint64_t>((static_cast<u128>(1) << 64) % Q);
-  constexpr uint64_t cs = static_cast<uint64_t>((static_cast<u128>(c) << 64) / Q);
-  constexpr uint64_t mu = ~0ull / Q;
-  const uint64_t h = static_cast<uint64_t>(x >> 64), l = static_cast<uint64_t>(x);
-  const uint64_t r1 = h * c - __umul64hi(h, cs) * Q;
-  const uint64_t r2 = l - __umul64hi(l, mu) * Q;
-  uint64_t r = r1 + r2;
-  r = min(r, r - 4 * Q);
-  r = min(r, r - 2 * Q);
-  return min(r, r - Q);
+// Recombination modulo q = 2^60 - c. Four classes at a time are exact in 64
+// bits: w(S) = S_0 + 2^8 S_1 + 2^16 S_2 + 2^24 S_3 < 2^56.
+__device__ __forceinline__ uint64_t four(uint32_t s0, uint32_t s1, uint32_t s2, uint32_t s3) {
+  return opir60::mad32(s3, 1u << 24, opir60::mad32(s2, 1u << 16, opir60::mad32(s1, 1u << 8, s0)));
 }
-
-// (lo + (hi mod q) 2^64) mod q for one limb
-template <uint64_t Q>
-__device__ __forceinline__ uint64_t combine(u128 lo, u128 hi) {
-  constexpr uint64_t c64 = static_cast<uint64_t>((static_cast<u128>(1) << 64) % Q);
-  const uint64_t h = red128_tc<Q>(hi);
-  return red128_tc<Q>(lo + static_cast<u128>(h) * c64);  // < 2^88 + 2^120
+// 2^32 x (mod q) for x < 2^60, below 2^60 + 2^49
+__device__ __forceinline__ uint64_t shl32(uint64_t x, uint32_t c) {
+  return opir60::mad32(static_cast<uint32_t>(x >> 28), c, (x & 0xFFFFFFFull) << 32);
+}
+// lo0 + 2^32 lo1 + 2^64 g mod q, g = hi0 + 2^32 hi1 below 2^61: 2^64 = 16 c
+// (mod q). The sum stays below 2^62; canonical. About 45 instructions an
+// output, where 128-bit sums and their two Barrett reductions took about 250:
+// with 32 columns there is one accumulator set, so the tensor cores wait for
+// them (N = 2048, batch 32 of 2^18 entries: 10.16 -> 9.93 ms a batch).
+__device__ __forceinline__ uint64_t combine(uint64_t lo0, uint64_t lo1, uint64_t g, uint32_t c) {
+  const uint64_t y = opir60::mul32(static_cast<uint32_t>(g >> 32), 16 * c);  // < 2^50
+  uint64_t r = opir60::mad32(static_cast<uint32_t>(g), 16 * c, lo0);
+  r += shl32(lo1, c) + shl32(y, c);
+  r = opir60::add64(r & opir60::kLow60, static_cast<uint32_t>(r >> 60) * c);
+  const uint64_t q = (1ull << 60) - c;
+  return min(r, r - q);
 }
 
 __global__ void __launch_bounds__(kThreadsTc, 1)
@@ -254,7 +254,7 @@ k4_scan_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
       }
       fence_after();
       const uint32_t ct = it % a.col_tiles, mt = (it / a.col_tiles) % a.m_tiles, z = it / per_z;
-      const bool limb1 = z >= static_cast<uint32_t>(kN);
+      const uint32_t fold_c = z >= static_cast<uint32_t>(kN) ? opir60::Fold<kQ1>::c : opir60::Fold<kQ0>::c;
       const uint32_t m = mt * kM + row;
       // cmat[z][column][row]: a warp's 32 rows of one column are contiguous
       uint64_t *dst = a.cmat + static_cast<uint64_t>(z) * a.ncols * a.other + m;
@@ -266,36 +266,27 @@ k4_scan_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUte
       for (int cc = 0; cc < 2; ++cc) {
         const uint32_t c0 = cbeg + 8 * cc;
         if (8 * cc >= static_cast<int>(nt / 2)) break;
-        u128 lo[8], hi[8];
-        {
-          uint32_t P[8][8];
-#pragma unroll
-          for (int s2 = 0; s2 < 8; ++s2) tmem_ld8(tbase + s2 * nt + c0, P[s2]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            u128 v = P[7][c];
-#pragma unroll
-            for (int s2 = 6; s2 >= 0; --s2) v = (v << 8) + P[s2][c];
-            lo[c] = v;
-          }
-        }
+        uint64_t g[8];
         {
           uint32_t P[7][8];
 #pragma unroll
           for (int s2 = 0; s2 < 7; ++s2) tmem_ld8(tbase + (8 + s2) * nt + c0, P[s2]);
           tmem_wait_ld();
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            u128 v = P[6][c];
-#pragma unroll
-            for (int s2 = 5; s2 >= 0; --s2) v = (v << 8) + P[s2][c];
-            hi[c] = v;
-          }
+          for (int c = 0; c < 8; ++c)
+            g[c] = four(P[0][c], P[1][c], P[2][c], P[3][c]) +
+                   shl32(four(P[4][c], P[5][c], P[6][c], 0), fold_c);
         }
+        {
+          uint32_t P[8][8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          outv[8 * cc + c] = limb1 ? combine<kQ1>(lo[c], hi[c]) : combine<kQ0>(lo[c], hi[c]);
+          for (int s2 = 0; s2 < 8; ++s2) tmem_ld8(tbase + s2 * nt + c0, P[s2]);
+          tmem_wait_ld();
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            outv[8 * cc + c] = combine(four(P[0][c], P[1][c], P[2][c], P[3][c]),
+                                       four(P[4][c], P[5][c], P[6][c], P[7][c]), g[c], fold_c);
+        }
       }
       // the accumulators are in registers: hand the TMEM set back first
       fence_before();
