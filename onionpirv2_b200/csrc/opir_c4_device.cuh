@@ -116,12 +116,13 @@ __device__ __forceinline__ void ld_plane(const uint64_t *pl, uint64_t (&v)[8], i
   for (int k = 0; k < 8; ++k) v[k] = pl[pad(posP<P>(t, k))];
 }
 
-// forward pass A on canonical inputs (A-order in registers)
-template <int L>
+// forward pass A (A-order in registers) on canonical inputs, or, Shifted, on
+// inputs between 192 c and 2q
+template <int L, bool Shifted = false>
 __device__ __forceinline__ void fA(uint64_t (&v)[8]) {
   ulonglong2 w[7];
   tw_const<L, true>(w, 1, 0);
-  opir60::fpass8<Limb<L>::q, true>(v, w);
+  opir60::fpass8<Limb<L>::q, !Shifted>(v, w);
 }
 // Forward passes B and C over np planes stored in A-order (after fA), up to
 // a __syncthreads; ends synchronised. Then: ld_plane<3> + fD.
@@ -212,14 +213,13 @@ __device__ __forceinline__ void iA(uint64_t (&v)[8]) {
 }
 
 // ------------------------------------------------------ RNS <-> integer
-// Garner compose of canonical limbs into [0, q0 q1) (gsw.cpp:22-53)
-__device__ __forceinline__ unsigned __int128 compose(uint64_t r0, uint64_t r1, uint64_t q0inv,
-                                                     uint64_t q0inv_sh) {
-  const uint64_t r0m = min(r0, r0 - kQ1);  // q0 < 2 q1
-  const uint64_t diff = r1 - r0m + kQ1;    // (0, 2 q1)
-  uint64_t s = mul_shoup<kQ1>(diff, q0inv, q0inv_sh);
+// Garner compose of canonical limbs into [0, q0 q1) (gsw.cpp:22-53); q0inv =
+// q0^-1 mod q1 (opir60::twiddle), q0 s = 2^60 s - c0 s
+__device__ __forceinline__ unsigned __int128 compose(uint64_t r0, uint64_t r1, ulonglong2 q0inv) {
+  uint64_t s = opir60::mul<kQ1>(r1 - r0 + 2 * kQ1, q0inv);  // r0 < q0 < 2 q1
   s = min(s, s - kQ1);
-  return static_cast<unsigned __int128>(kQ0) * s + r0;
+  using u128 = unsigned __int128;
+  return (static_cast<u128>(s) << 60) + r0 - static_cast<u128>(s) * opir60::Fold<kQ0>::c;
 }
 
 }  // namespace opir4

@@ -379,18 +379,16 @@ __device__ __forceinline__ void expand_body(const Dev4 &P, uint32_t galois_inv, 
       const uint32_t src = w & (kN - 1);
       uint64_t a0 = ct[2 * kN + src], a1 = ct[3 * kN + src];
       if (neg) { a0 = neg_mod<kQ0>(a0); a1 = neg_mod<kQ1>(a1); }
-      u[k] = bv_digit_source<kLKs, kBaseKs>(compose(a0, a1, P.q0inv, P.q0inv_sh));
+      u[k] = bv_digit_source<kLKs, kBaseKs>(compose(a0, a1, P.q0inv));
     }
 #pragma unroll
     for (int e = 0; e < kExpGroup; ++e) {
       uint64_t v[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int64_t r = static_cast<int64_t>(field<kBaseKs>(u[k], g * kExpGroup + e)) -
-                          ((1ll << (kBaseKs - 1)) - 1);
-        v[k] = r >= 0 ? static_cast<uint64_t>(r) : static_cast<uint64_t>(r + static_cast<int64_t>(Q));
+        v[k] = field<kBaseKs>(u[k], g * kExpGroup + e) + (Q - ((1ull << (kBaseKs - 1)) - 1));
       }
-      fA<L>(v);
+      fA<L, true>(v);
       st_plane<0>(sm4 + e * kPad, v, tid);
     }
     __syncthreads();
@@ -510,18 +508,16 @@ __device__ __forceinline__ void expand_split_body(const Dev4 &P, uint32_t galois
       const uint32_t src = w & (kN - 1);
       uint64_t a0 = ct[2 * kN + src], a1 = ct[3 * kN + src];
       if (neg) { a0 = neg_mod<kQ0>(a0); a1 = neg_mod<kQ1>(a1); }
-      u[k] = bv_digit_source<kLKs, kBaseKs>(compose(a0, a1, P.q0inv, P.q0inv_sh));
+      u[k] = bv_digit_source<kLKs, kBaseKs>(compose(a0, a1, P.q0inv));
     }
 #pragma unroll
     for (int e = 0; e < D; ++e) {
       uint64_t v[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int64_t r = static_cast<int64_t>(field<kBaseKs>(u[k], rank * D + e)) -
-                          ((1ll << (kBaseKs - 1)) - 1);
-        v[k] = r >= 0 ? static_cast<uint64_t>(r) : static_cast<uint64_t>(r + static_cast<int64_t>(Q));
+        v[k] = field<kBaseKs>(u[k], rank * D + e) + (Q - ((1ull << (kBaseKs - 1)) - 1));
       }
-      fA<L>(v);
+      fA<L, true>(v);
       st_plane<0>(sm4 + e * kPad, v, tid);
     }
   }
@@ -625,7 +621,7 @@ __device__ __forceinline__ void gadget_mac(const Dev4 &P, const uint64_t *x, con
           v0 = sub_mod<kQ0>(y[p * 2 * kN + j], v0);
           v1 = sub_mod<kQ1>(y[p * 2 * kN + kN + j], v1);
         }
-        u[k] = compose(v0, v1, P.q0inv, P.q0inv_sh);
+        u[k] = compose(v0, v1, P.q0inv);
       }
 #pragma unroll
       for (int e = 0; e < G; ++e) {
@@ -959,7 +955,7 @@ __device__ __forceinline__ void gadget_part(const Dev4 &P, const uint64_t *x, co
       const int j = posA(tid, k);
       const uint64_t v0 = sub_mod<kQ0>(y[p * 2 * kN + j], x[p * 2 * kN + j]);
       const uint64_t v1 = sub_mod<kQ1>(y[p * 2 * kN + kN + j], x[p * 2 * kN + kN + j]);
-      u[k] = compose(v0, v1, P.q0inv, P.q0inv_sh);
+      u[k] = compose(v0, v1, P.q0inv);
     }
     for (int e = 0; e < dn; ++e) {
       uint64_t v[8];
@@ -1081,7 +1077,7 @@ k4_modswitch(Dev4 P, const uint64_t *__restrict__ ct_all, uint64_t ct_stride,
   const uint64_t *ct = ct_all + static_cast<uint64_t>(b) * ct_stride * kCtWords;
   for (int idx = blockIdx.y * blockDim.x + threadIdx.x; idx < 2 * kN; idx += gridDim.y * blockDim.x) {
     const int p = idx >> 12, j = idx & (kN - 1);
-    const u128 x = compose(ct[p * 2 * kN + j], ct[p * 2 * kN + kN + j], P.q0inv, P.q0inv_sh);
+    const u128 x = compose(ct[p * 2 * kN + j], ct[p * 2 * kN + kN + j], P.q0inv);
     uint64_t v = static_cast<uint64_t>((x + (static_cast<u128>(kQ1) >> 1)) / kQ1);
     if (v >= kQ0) v -= kQ0;
     const uint64_t r = rescale_dev(v, kQ0, P.small_q);

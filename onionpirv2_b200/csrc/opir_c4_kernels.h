@@ -35,7 +35,7 @@ struct Tables {
 };
 
 struct Dev4 {
-  uint64_t q0inv, q0inv_sh;        // q0^-1 mod q1 and its Shoup companion
+  ulonglong2 q0inv;                // q0^-1 mod q1 (opir60::twiddle)
   Tables T;
   uint64_t small_q;
   uint32_t small_q_width;

@@ -191,8 +191,7 @@ void Server::setup_c4_tables() {
   const ulonglong2 ninv[2] = {opir60::twiddle(t[0].n_inv, t[0].q), opir60::twiddle(t[1].n_inv, t[1].q)};
   const ulonglong2 w1n[2] = {opir60::twiddle(t[0].w1_ninv, t[0].q), opir60::twiddle(t[1].w1_ninv, t[1].q)};
   upload_constants(fw, iw, ninv, w1n);
-  dp_.q0inv = p_.q1_inv_mod_q2;
-  dp_.q0inv_sh = static_cast<uint64_t>((static_cast<unsigned __int128>(dp_.q0inv) << 64) / kQ1);
+  dp_.q0inv = opir60::twiddle(p_.q1_inv_mod_q2, kQ1);
 }
 
 // ------------------------------------------------------------------ launches

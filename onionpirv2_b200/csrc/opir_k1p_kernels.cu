@@ -108,9 +108,8 @@ __device__ __forceinline__ uint64_t digit_source(uint64_t v) {
   return v + C - (v > kQ / 2 ? kQ : 0);
 }
 template <int B>
-__device__ __forceinline__ uint64_t digit_res(uint64_t u, int i) {  // r_i mod q
-  const int64_t r = static_cast<int64_t>((u >> (B * i)) & ((1ull << B) - 1)) - (1ll << (B - 1));
-  return r >= 0 ? static_cast<uint64_t>(r) : static_cast<uint64_t>(r + static_cast<int64_t>(kQ));
+__device__ __forceinline__ uint64_t digit_res(uint64_t u, int i) {  // q + r_i
+  return ((u >> (B * i)) & ((1ull << B) - 1)) + (kQ - (1ull << (B - 1)));
 }
 
 // ------------------------------------------------------------ NTT
@@ -137,11 +136,13 @@ __device__ __forceinline__ void ld_plane(const uint64_t *pl, uint64_t (&v)[8], i
   }
 }
 
-// pass A (stages 1-3), canonical input
+// pass A (stages 1-3) on canonical inputs, or, Shifted, on inputs between
+// 192 c and 2q
+template <bool Shifted = false>
 __device__ __forceinline__ void fA(uint64_t (&v)[8]) {
   const ulonglong2 w[7] = {c1_fwt[1], c1_fwt[2], c1_fwt[3], c1_fwt[4],
                            c1_fwt[5], c1_fwt[6], c1_fwt[7]};
-  opir60::fpass8<kQ, true>(v, w);
+  opir60::fpass8<kQ, !Shifted>(v, w);
 }
 __device__ __forceinline__ void load_b(ulonglong2 (&w)[7], const ulonglong2 *c, int t) {
   const int g = t >> 5;
@@ -487,7 +488,7 @@ __device__ __forceinline__ void expand_body(const Dev1 &P, uint32_t galois_inv, 
       uint64_t v[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) v[k] = digit_res<kBaseKs>(u[k], g * kGroup + e);
-      fA(v);
+      fA<true>(v);
       st_plane<0>(sm1 + e * kPad, v, tid);
     }
     __syncthreads();
@@ -594,7 +595,7 @@ __device__ __forceinline__ void gadget_mac(const Dev1 &P, const uint64_t *x, con
         uint64_t v[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) v[k] = digit_res<B>(u[k], g * G + e);
-        fA(v);
+        fA<true>(v);
         st_plane<0>(sm + e * kPad, v, tid);
       }
       __syncthreads();
