@@ -64,16 +64,6 @@ int sm_count() {
   return n;
 }
 
-// Cluster-split levels (k4_expand_level_split, k4_mux_level_split): on
-// unless OPIR_SPLIT=0.
-bool split_enabled() {
-  static const bool on = [] {
-    const char *e = std::getenv("OPIR_SPLIT");
-    return !(e && std::strcmp(e, "0") == 0);
-  }();
-  return on;
-}
-
 // Launch with a 1-D cluster of `c` CTAs along x.
 template <typename Kern, typename... Args>
 void launch_cluster(Kern kernel, int c, dim3 grid, size_t smem, cudaStream_t st, const char *what,
@@ -1100,6 +1090,16 @@ k4_modswitch(Dev4 P, const uint64_t *__restrict__ ct_all, uint64_t ct_stride,
 }  // namespace
 
 // ============================================================== launchers
+// Cluster-split levels (expansion and MUX, both 64-bit-limb sets): on unless
+// OPIR_SPLIT=0.
+bool split_enabled() {
+  static const bool on = [] {
+    const char *e = std::getenv("OPIR_SPLIT");
+    return !(e && std::strcmp(e, "0") == 0);
+  }();
+  return on;
+}
+
 uint64_t launch_count() { return g_launches4.load(std::memory_order_relaxed); }
 void note_launches(int64_t delta) {
   g_launches4.fetch_add(static_cast<uint64_t>(delta), std::memory_order_relaxed);

@@ -47,6 +47,7 @@ struct Shape4 {
 };
 
 uint64_t launch_count();
+bool split_enabled();
 // Adjusts the launch counter (a launch made outside opir_c4_kernels.cu, or
 // kernels replayed from a CUDA graph).
 void note_launches(int64_t delta);

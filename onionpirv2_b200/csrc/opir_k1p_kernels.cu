@@ -19,6 +19,8 @@
 #include <stdexcept>
 #include <string>
 
+#include <cooperative_groups.h>
+
 namespace opir1 {
 
 namespace {
@@ -542,8 +544,116 @@ __device__ __forceinline__ void expand_body(const Dev1 &P, uint32_t galois_inv, 
   }
 }
 
-// MINB CTAs per SM: 2 (128 registers, a few spilled) when a level fills
-// the GPU twice over, else 1 (no spills, lower latency per CTA).
+// The two output polynomials' folded partial sums of a cluster's CTAs meet in
+// distributed shared memory: CTA 0 gets polynomial 0's total, CTA 1
+// polynomial 1's, folded and INTT'd (A order, canonical); the others return
+// false. ex: 16 kThreads words of shared memory, free of other use.
+template <int C>
+__device__ __forceinline__ bool cluster_total(const Dev1 &P, uint64_t *ex, int rank,
+                                              const uint64_t (&acc0)[8], const uint64_t (&acc1)[8],
+                                              uint64_t (&v)[8]) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    ex[k * kThreads + tid] = acc0[k];
+    ex[(8 + k) * kThreads + tid] = acc1[k];
+  }
+  cluster.sync();
+  if (rank < 2) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = rank == 0 ? acc0[k] : acc1[k];
+    for (int r = 0; r < C; ++r) {
+      if (r == rank) continue;
+      const uint64_t *rex = cluster.map_shared_rank(ex, r);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] += rex[(rank * 8 + k) * kThreads + tid];
+    }
+  }
+  cluster.sync();  // every remote read is done before shared memory is reused
+  if (rank >= 2) return false;
+  ulonglong2 wd[6];
+  load_d(wd, P.iwt, tid);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = opir60::fold<kQ>(v[k]);  // C (q + 16 c) < 2^64
+  iD(v, wd);
+  st_plane<3>(ex, v, tid);
+  __syncthreads();
+  inv_mid(ex, 1, P.iwt);
+  ld_plane<0>(ex, v, tid);
+  iA(v);
+  return true;
+}
+
+// Expansion level, cluster split: with few nodes each node's key switch runs
+// on a cluster of C CTAs. CTA r transforms digits [r D, (r + 1) D) (D = L_KS /
+// C) of sigma_k(c1) and multiplies them with the key rows; CTA 0 finishes the
+// b part (c0 of both children), CTA 1 the a part. Same children bit for bit.
+template <int C>
+__global__ void __launch_bounds__(kThreads, 2)
+k1p_expand_level_split(Dev1 P, uint32_t galois_inv, uint32_t kshift,
+                       const uint64_t *__restrict__ in, uint64_t in_stride,
+                       uint64_t *__restrict__ out, uint64_t out_stride,
+                       const uint64_t *const *__restrict__ bv_keys, uint64_t bv_level_off) {
+  static_assert(kLKs % C == 0 && kLKs / C <= kGroup, "digits per CTA fit the planes");
+  constexpr int D = kLKs / C;
+  extern __shared__ uint64_t sm1[];
+  const int rank = static_cast<int>(cooperative_groups::this_cluster().block_rank());
+  const int node = blockIdx.x / C, b = blockIdx.z, tid = threadIdx.x;
+  const uint64_t *ct = in + (static_cast<uint64_t>(b) * in_stride + node) * kCtWords;
+  const uint64_t *key = bv_keys[b] + bv_level_off;
+  {
+    uint64_t u[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const uint32_t j = posA(tid, k);
+      const uint32_t w = (j * galois_inv) & (2 * kN - 1);
+      const uint64_t a = ct[kN + (w & (kN - 1))];
+      u[k] = digit_source<kLKs, kBaseKs>(w >= kN ? neg_q(a) : a);  // sigma_k(c1)
+    }
+#pragma unroll
+    for (int e = 0; e < D; ++e) {
+      uint64_t v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = digit_res<kBaseKs>(u[k], rank * D + e);
+      fA<true>(v);
+      st_plane<0>(sm1 + e * kPad, v, tid);
+    }
+  }
+  __syncthreads();
+  fwd_mid(sm1, D, P.fwt);
+  uint64_t ab[8], aa[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) ab[k] = aa[k] = 0;
+  mac_group(P, sm1, D, key + static_cast<uint64_t>(rank) * D * kCtWords, kCtWords, ab, aa, tid);
+  __syncthreads();
+  uint64_t dv[8];
+  if (!cluster_total<C>(P, sm1, rank, ab, aa, dv)) return;
+  uint64_t *outL = out + (static_cast<uint64_t>(b) * out_stride + 2ull * node) * kCtWords + rank * kN;
+  uint64_t *outR = outL + kCtWords;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const uint32_t j = posA(tid, k);
+    uint64_t nv = dv[k];
+    if (rank == 0) {  // c0' = sigma_k(c0) + delta_b
+      const uint32_t w = (j * galois_inv) & (2 * kN - 1);
+      const uint64_t z = ct[w & (kN - 1)];
+      nv = add_q(w >= kN ? neg_q(z) : z, nv);
+    }
+    const uint64_t o = ct[rank * kN + j];
+    outL[j] = add_q(o, nv);
+    const uint64_t dd = sub_q(o, nv);
+    int dst = static_cast<int>(j) - static_cast<int>(kshift);
+    const bool wrap = dst < 0;
+    if (wrap) dst += kN;
+    outR[dst] = wrap ? neg_q(dd) : dd;
+  }
+}
+
+// MINB CTAs per SM: 2 (128 registers, a few spilled) when a level has more
+// CTAs than SMs, so that up to twice as many run in one wave, else 1 (no
+// spills, lower latency per CTA).
 template <int MINB>
 __global__ void __launch_bounds__(kThreads, MINB)
 k1p_expand_level(Dev1 P, uint32_t galois_inv, uint32_t kshift, const uint64_t *__restrict__ in,
@@ -846,6 +956,62 @@ k1p_mux_level(Dev1 P, Shape1 S, uint32_t level, uint32_t n_pairs, uint32_t offse
   }
 }
 
+// MUX level, cluster split: with few pairs each MUX runs on a cluster of C
+// CTAs. CTA r takes digits [d0, d0 + dn) of polynomial p of y - x (C = 2: p =
+// r, all l digits; C = 4: p = r / 2, digits 0-2 or 3-4); CTAs 0 and 1 finish
+// output polynomial c0 / c1. Pair i reads x = in[i xs], y = in[i xs + yoff]
+// and writes out[i]. Bit for bit the single-CTA MUX.
+template <int C>
+__global__ void __launch_bounds__(kThreads, 2)
+k1p_mux_level_split(Dev1 P, Shape1 S, uint32_t level, uint32_t xs, uint32_t yoff,
+                    const uint64_t *__restrict__ in, uint64_t *__restrict__ out,
+                    uint64_t mid_stride, const uint64_t *__restrict__ sel) {
+  static_assert(C == 2 || C == 4, "cluster of 2 or 4 CTAs");
+  extern __shared__ uint64_t sm1[];
+  const int rank = static_cast<int>(cooperative_groups::this_cluster().block_rank());
+  const int b = blockIdx.z, tid = threadIdx.x;
+  const uint32_t i = blockIdx.x / C;
+  const uint64_t *x = in + (static_cast<uint64_t>(b) * mid_stride + static_cast<uint64_t>(i) * xs) * kCtWords;
+  const uint64_t *y = x + static_cast<uint64_t>(yoff) * kCtWords;
+  const uint64_t *rgsw =
+      sel + (static_cast<uint64_t>(b) * (S.num_dims - 1) + level) * 2 * kLEp * kCtWords;
+  constexpr int kHalf = (kLEp + 1) / 2;
+  const int p = C == 2 ? rank : rank >> 1;
+  const int d0 = C == 2 ? 0 : (rank & 1) * kHalf;
+  const int dn = C == 2 ? kLEp : ((rank & 1) ? kLEp - kHalf : kHalf);
+  {
+    uint64_t u[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int j = posA(tid, k);
+      u[k] = digit_source<kLEp, kBaseEp>(sub_q(y[p * kN + j], x[p * kN + j]));
+    }
+    for (int e = 0; e < dn; ++e) {
+      uint64_t v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = digit_res<kBaseEp>(u[k], d0 + e);
+      fA<true>(v);
+      st_plane<0>(sm1 + e * kPad, v, tid);
+    }
+  }
+  __syncthreads();
+  fwd_mid<false>(sm1, dn, P.fwt);
+  uint64_t acc0[8], acc1[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) acc0[k] = acc1[k] = 0;
+  mac_group(P, sm1, dn, rgsw + static_cast<uint64_t>(p * kLEp + kLEp - 1 - d0) * kCtWords,
+            -static_cast<int64_t>(kCtWords), acc0, acc1, tid);
+  __syncthreads();
+  uint64_t v[8];
+  if (!cluster_total<C>(P, sm1, rank, acc0, acc1, v)) return;
+  uint64_t *o = out + (static_cast<uint64_t>(b) * mid_stride + i) * kCtWords + rank * kN;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int j = posA(tid, k);
+    o[j] = add_q(x[rank * kN + j], v[k]);
+  }
+}
+
 // ------------------------------------------------------------ modulus switch
 // mod_switch_inplace (server.cpp:1025-1043) with utils::rescale
 // (utils.cpp:445-462): centred round(v small_q / q), then the response bit
@@ -916,6 +1082,41 @@ void launch_db_preprocess(const Dev1 &P, const Shape1 &s, const uint64_t *coeffs
   check_launch("k1p_db_preprocess");
 }
 
+namespace {
+// CTAs per item of a level of `ctas` items: the widest cluster of 2, 4 or 8
+// (at most `widest`) with which the level is still one wave of two CTAs an SM.
+// A level's latency is that of one CTA's chain of transforms: a lone query of
+// 2^15 entries 620 -> 378 us, of 2^18 1172 -> 923, batch 4 1683 -> 1498, batch
+// 32 9690 -> 9595; with one CTA an SM as the line 384, 939, 1506, 9615.
+int split_of(uint64_t ctas, int widest) {
+  if (!opir4::split_enabled()) return 1;
+  int c = widest;
+  while (c > 1 && c * ctas > 2ull * sms()) c /= 2;
+  return c;
+}
+
+template <typename Kern, typename... Args>
+void launch_cluster(Kern kernel, int c, dim3 grid, size_t smem, cudaStream_t st, const char *what,
+                    Args... args) {
+  set_smem(kernel, smem);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = c;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
+  check_launch(what);
+}
+}  // namespace
+
 void launch_expand_level(const Dev1 &P, const Shape1 &s, uint32_t d, const uint64_t *in,
                          uint64_t in_stride, uint64_t *out, uint64_t out_stride,
                          const uint64_t *const *bv_keys, uint64_t bv_level_stride, uint32_t batch,
@@ -932,7 +1133,7 @@ void launch_expand_level(const Dev1 &P, const Shape1 &s, uint32_t d, const uint6
     throw std::invalid_argument("NTT-form children only at the last expansion level");
   if (ntt_nodes > 0) {
     const dim3 grid(ntt_nodes, 1, batch);
-    if (static_cast<uint64_t>(ntt_nodes) * batch >= 2ull * sms()) {
+    if (static_cast<uint64_t>(ntt_nodes) * batch > static_cast<uint64_t>(sms())) {
       set_smem(k1p_expand_level_ntt<2>, smem);
       k1p_expand_level_ntt<2><<<grid, kThreads, smem, st>>>(P, galois, galois_inv, k, in,
                                                              in_stride, out, out_stride, bv_keys,
@@ -947,8 +1148,23 @@ void launch_expand_level(const Dev1 &P, const Shape1 &s, uint32_t d, const uint6
   }
   const uint32_t rest = nodes - ntt_nodes;  // coefficient-form children
   if (rest == 0) return;
+  const uint64_t ctas = static_cast<uint64_t>(rest) * batch;
+  const int split = ntt_nodes ? 1 : split_of(ctas, 8);
+  if (split > 1) {
+    const dim3 g(rest * split, 1, batch);
+    if (split == 8)
+      launch_cluster(k1p_expand_level_split<8>, 8, g, smem, st, "k1p_expand_level_split", P, galois_inv, k,
+                     in, in_stride, out, out_stride, bv_keys, koff);
+    else if (split == 4)
+      launch_cluster(k1p_expand_level_split<4>, 4, g, smem, st, "k1p_expand_level_split", P, galois_inv, k,
+                     in, in_stride, out, out_stride, bv_keys, koff);
+    else
+      launch_cluster(k1p_expand_level_split<2>, 2, g, smem, st, "k1p_expand_level_split", P, galois_inv, k,
+                     in, in_stride, out, out_stride, bv_keys, koff);
+    return;
+  }
   const dim3 grid(rest, 1, batch);
-  if (static_cast<uint64_t>(rest) * batch >= 2ull * sms()) {
+  if (ctas > static_cast<uint64_t>(sms())) {
     set_smem(k1p_expand_level<2>, smem);
     k1p_expand_level<2><<<grid, kThreads, smem, st>>>(P, galois_inv, k, in, in_stride, out,
                                                        out_stride, bv_keys, koff, ntt_nodes);
@@ -1033,6 +1249,19 @@ void launch_mux_level(const Dev1 &P, const Shape1 &s, uint32_t level, uint32_t t
     n_pairs = half;
   }
   const size_t smem = plane_bytes(kLEp);
+  const int split = copies ? 1 : split_of(static_cast<uint64_t>(n_pairs) * batch, 4);
+  if (split > 1) {
+    // offset == copies == 0 here, so level 0 pairs (2i, 2i + 1) into i
+    const uint32_t xs = level == 0 ? 2 : 1, yoff = level == 0 ? 1 : half;
+    const dim3 g(n_pairs * split, 1, batch);
+    if (split == 4)
+      launch_cluster(k1p_mux_level_split<4>, 4, g, smem, st, "k1p_mux_level_split", P, s, level, xs, yoff,
+                     in, out, mid_stride, sel);
+    else
+      launch_cluster(k1p_mux_level_split<2>, 2, g, smem, st, "k1p_mux_level_split", P, s, level, xs, yoff,
+                     in, out, mid_stride, sel);
+    return;
+  }
   set_smem(k1p_mux_level, smem);
   k1p_mux_level<<<dim3(n_pairs + copies, 1, batch), kThreads, smem, st>>>(
       P, s, level, n_pairs, offset, half, in, out, mid_stride, sel);

@@ -57,3 +57,19 @@ def test_extreme_residues_match_oracle(name, query, keys):
     want_sel = ref.complete_selectors(want)
     assert np.array_equal(srv.complete_selectors(1, got).reshape(want_sel.shape), want_sel)
     assert np.array_equal(srv.make_query(1, q), ref.make_query(q))
+
+
+@pytest.mark.parametrize("batch", [2, 5, 10, 19, 38, 75])
+def test_k1p_batches_match_lone_queries(batch):
+    """Lone queries run every level on clusters of CTAs; growing batches leave
+    the 8-, 4- and 2-CTA forms one after the other for one CTA an item."""
+    op, cl, srv, ref = setup("k1p")
+    bv, gsw = cl.bv_keys(), cl.gsw_key()
+    srv.set_client_keys(1, bv, gsw)
+    ref.set_keys(bv, gsw)
+    qs = [cl.query(i) for i in (0, 21, 42)]
+    want = np.stack([ref.make_query(q) for q in qs])
+    assert np.array_equal(np.stack([srv.make_query(1, q) for q in qs]), want)
+    pick = np.arange(batch) % 3
+    got = srv.make_query_batch([1] * batch, np.stack([qs[i] for i in pick]))
+    assert np.array_equal(got, want[pick])
