@@ -868,7 +868,8 @@ k1p_fst_pack(const uint64_t *__restrict__ qm, uint64_t q_stride, uint64_t p_stri
 // rows of one column.
 constexpr int kEpiRows = 4;
 
-__global__ void __launch_bounds__(kThreads)
+template <bool VEC>
+__global__ void __launch_bounds__(kThreads, 2)
 k1p_epilogue(Dev1 P, Shape1 S, const uint64_t *__restrict__ cmat, uint32_t ncols,
              uint64_t *__restrict__ mid, uint64_t mid_stride) {
   extern __shared__ uint64_t sm1[];
@@ -880,8 +881,14 @@ k1p_epilogue(Dev1 P, Shape1 S, const uint64_t *__restrict__ cmat, uint32_t ncols
     for (int k = 0; k < 8; ++k) {
       const uint64_t z = posD(tid, k);
       const uint64_t *src = cmat + (z * ncols + c) * S.other + r0;
+      if (VEC && r0 + kEpiRows <= S.other) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(src);
+        const ulonglong2 d = *reinterpret_cast<const ulonglong2 *>(src + 2);
+        v[0][k] = a.x; v[1][k] = a.y; v[2][k] = d.x; v[3][k] = d.y;
+      } else {
 #pragma unroll
-      for (int e = 0; e < kEpiRows; ++e) v[e][k] = r0 + e < S.other ? src[e] : 0;
+        for (int e = 0; e < kEpiRows; ++e) v[e][k] = r0 + e < S.other ? src[e] : 0;
+      }
     }
     ulonglong2 wd[6];
     load_d(wd, P.iwt, tid);
@@ -1223,10 +1230,16 @@ void launch_fst_pack_leaves(const Shape1 &s, const uint64_t *leaves, uint64_t le
 void launch_epilogue(const Dev1 &P, const Shape1 &s, const uint64_t *cmat, uint64_t *mid,
                      uint64_t mid_stride, uint32_t batch, cudaStream_t st) {
   const size_t smem = plane_bytes(kEpiRows);
-  set_smem(k1p_epilogue, smem);
   const uint32_t ncols = 2 * batch;
-  k1p_epilogue<<<dim3((s.other + kEpiRows - 1) / kEpiRows, 1, ncols), kThreads, smem, st>>>(
-      P, s, cmat, ncols, mid, mid_stride);
+  const dim3 grid((s.other + kEpiRows - 1) / kEpiRows, 1, ncols);
+  // an even row count keeps every 4-row group (r0 a multiple of 4) 16-byte aligned
+  if (s.other % 2 == 0) {
+    set_smem(k1p_epilogue<true>, smem);
+    k1p_epilogue<true><<<grid, kThreads, smem, st>>>(P, s, cmat, ncols, mid, mid_stride);
+  } else {
+    set_smem(k1p_epilogue<false>, smem);
+    k1p_epilogue<false><<<grid, kThreads, smem, st>>>(P, s, cmat, ncols, mid, mid_stride);
+  }
   check_launch("k1p_epilogue");
 }
 
