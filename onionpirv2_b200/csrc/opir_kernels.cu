@@ -936,6 +936,23 @@ k_scan(DevParams P, uint32_t n0, uint32_t n0p, uint32_t m, const uint8_t *__rest
 }
 
 // ----------------------------------------------------------- scan epilogue
+// Eight words from any word of a 16-byte aligned buffer of whole 16-byte
+// chunks: the two or three chunks that hold them, shifted into place. Eight
+// scalar loads a level made the epilogue of a 683-row database 342 us a batch
+// of 13, this 236.
+__device__ __forceinline__ void ld8_window(const uint32_t *src, uint32_t (&w)[8]) {
+  const uint32_t off = (reinterpret_cast<uintptr_t>(src) >> 2) & 3;
+  const uint4 *p = reinterpret_cast<const uint4 *>(src - off);
+  const uint4 a = __ldg(p), b = __ldg(p + 1);
+  const uint4 c = off ? __ldg(p + 2) : make_uint4(0, 0, 0, 0);
+  const uint32_t x[11] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z};
+  uint32_t y[9];
+#pragma unroll
+  for (int i = 0; i < 9; ++i) y[i] = (off & 2) ? x[i + 2] : x[i];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) w[i] = (off & 1) ? y[i + 1] : y[i];
+}
+
 // inter_to_cts_composite (server.cpp:529-597): INTT of every candidate of
 // the scan. cmat is [residue x level][column][row]; a block transforms 8
 // adjacent rows of one column and one residue, so the 8 words it reads per
@@ -957,6 +974,11 @@ __device__ __forceinline__ void scan_epilogue_body(const DevParams &P, const Sha
       const uint4 hi = __ldg(reinterpret_cast<const uint4 *>(src + 4));
       v[0][k] = lo.x; v[1][k] = lo.y; v[2][k] = lo.z; v[3][k] = lo.w;
       v[4][k] = hi.x; v[5][k] = hi.y; v[6][k] = hi.z; v[7][k] = hi.w;
+    } else if (!VEC && r0 + 8 <= S.other) {
+      uint32_t w[8];
+      ld8_window(src, w);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e][k] = w[e];
     } else {
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e][k] = r0 + e < S.other ? __ldg(src + e) : 0u;
