@@ -209,7 +209,8 @@ def ntt_butterflies(params) -> dict:
     (L_KS digit NTTs + 2 INTTs, bv_keyswitch.cpp:296-367 / 373-481; nodes of
     level d = ceil(useful / 2^(h-d)), server.cpp:786-792); other dimensions =
     other_dim_sz - 1 external products (2 L_EP digit NTTs + 2 INTTs,
-    gsw.cpp:119-250, server.cpp:652-722). One butterfly = one Shoup product."""
+    gsw.cpp:119-250, server.cpp:652-722). One butterfly = one
+    product by a twiddle."""
     N = params.N
     per_ntt = (N // 2) * (N.bit_length() - 1)
     # NTTs run per residue (k1_comp) or RNS limb; CONFIG_N2048_K1 has one prime
@@ -226,7 +227,7 @@ def int_pipe_roofline(params, config: str, stages: dict, batch: int, device: int
     against the device's measured butterfly rate (register-resident probe)."""
     from onionpirv2_b200.server import measure_butterfly_rate
     peak = measure_butterfly_rate(config, device) / 1e9
-    out = {"bound": "integer multiply pipe (NTT butterflies, one Shoup product each)",
+    out = {"bound": "integer multiply pipe (NTT butterflies, one product by a twiddle each)",
            "unit": "Gbutterflies/s", "peak": peak,
            "peak_source": "measured (opir_measure_butterfly_rate: the kernels' radix-8 pass on "
                           "register operands, all SMs)", "stages": {}}
@@ -1076,19 +1077,17 @@ def bench_client(args, world, rank, local):
     tensor_path = (n >= 32 and os.environ.get("OPIR_CLIENT_TC", "1") != "0"
                    and os.environ.get("OPIR_CLIENT_WINDOW", "1") != "0")
     if tensor_path:
-        # tcgen05 byte-plane scans: 4 A planes x 4 x planes of N x N per response
-        # and scan (one scan mod small_q < 2^29; else two 25-bit halves of c1,
-        # each mod two primes: four scans)
-        scans = 1 if sq < (1 << 29) else 4
-        ops = n * scans * 2 * N * N * 16
+        # one exact tcgen05 product: the N x N secret matrix (one byte plane)
+        # by the byte planes of small_q
+        planes = (sq.bit_length() + 7) // 8
+        ops = n * 2 * N * N * planes
         peaks = measured_peaks()
         bf16 = peaks.get("bf16_tflops")
         peak = 2 * bf16 if bf16 else 2 * 1590.0   # int8 dense = 2 x bf16 dense
         achieved = ops / (ms_dec / 1e3) / 1e12
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TOP/s (int8)",
                 "frac": achieved / peak, "traffic": None,
-                "work": f"{scans} scan(s) x 2 N^2 x 16 byte-plane products per response "
-                        "(one secret plane is nonzero)",
+                "work": f"2 N^2 x {planes} byte-plane products per response",
                 "peak_kind": ("2 x measured" if bf16 else "2 x fallback")
                              + " dense bf16 (int8 dense is twice bf16 on B200)"}
     else:

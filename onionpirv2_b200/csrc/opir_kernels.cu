@@ -957,7 +957,8 @@ __device__ __forceinline__ void ld8_window(const uint32_t *src, uint32_t (&w)[8]
 // the scan. cmat is [residue x level][column][row]; a block transforms 8
 // adjacent rows of one column and one residue, so the 8 words it reads per
 // level are one contiguous 32-byte sector.
-template <int RES, bool VEC>
+enum class Rows { kScalar, kWindow, kAligned };  // how eight rows of a level are read
+template <int RES, Rows HOW>
 __device__ __forceinline__ void scan_epilogue_body(const DevParams &P, const Shape &S,
                                                    const uint32_t *cmat, uint32_t ncols,
                                                    uint32_t *mid, uint64_t mid_stride) {
@@ -969,12 +970,12 @@ __device__ __forceinline__ void scan_epilogue_body(const DevParams &P, const Sha
 #pragma unroll
   for (int k = 0; k < 8; ++k) {
     const uint32_t *src = cmat + (((uint64_t)RES * kN + posD(tid, k)) * ncols + c) * S.other + r0;
-    if (VEC && r0 + 8 <= S.other) {
+    if (HOW == Rows::kAligned && r0 + 8 <= S.other) {
       const uint4 lo = __ldg(reinterpret_cast<const uint4 *>(src));
       const uint4 hi = __ldg(reinterpret_cast<const uint4 *>(src + 4));
       v[0][k] = lo.x; v[1][k] = lo.y; v[2][k] = lo.z; v[3][k] = lo.w;
       v[4][k] = hi.x; v[5][k] = hi.y; v[6][k] = hi.z; v[7][k] = hi.w;
-    } else if (!VEC && r0 + 8 <= S.other) {
+    } else if (HOW == Rows::kWindow && r0 + 8 <= S.other) {
       uint32_t w[8];
       ld8_window(src, w);
 #pragma unroll
@@ -1008,14 +1009,14 @@ __device__ __forceinline__ void scan_epilogue_body(const DevParams &P, const Sha
   }
 }
 
-template <bool VEC>
+template <Rows HOW>
 __global__ void __launch_bounds__(kThreads, 2)
 k_scan_epilogue(DevParams P, Shape S, const uint32_t *__restrict__ cmat, uint32_t ncols,
                 uint32_t *__restrict__ mid, uint64_t mid_stride) {
   if (blockIdx.y == 0)
-    scan_epilogue_body<0, VEC>(P, S, cmat, ncols, mid, mid_stride);
+    scan_epilogue_body<0, HOW>(P, S, cmat, ncols, mid, mid_stride);
   else
-    scan_epilogue_body<1, VEC>(P, S, cmat, ncols, mid, mid_stride);
+    scan_epilogue_body<1, HOW>(P, S, cmat, ncols, mid, mid_stride);
 }
 
 // ------------------------------------------- first dimension row by row
@@ -1757,13 +1758,17 @@ void launch_scan_epilogue(const DevParams &P, const Shape &s, const uint32_t *cm
   const size_t smem = 8 * kPad * sizeof(uint32_t);
   const uint32_t ncols = 2 * batch;
   dim3 grid((s.other + 7) / 8, 2, ncols);
-  if (s.other % 4 == 0) {
-    set_smem(k_scan_epilogue<true>, smem);
-    k_scan_epilogue<true><<<grid, kThreads, smem, st>>>(P, s, cmat, ncols, mid, mid_stride);
-  } else {
-    set_smem(k_scan_epilogue<false>, smem);
-    k_scan_epilogue<false><<<grid, kThreads, smem, st>>>(P, s, cmat, ncols, mid, mid_stride);
-  }
+  const auto run = [&](auto kern) {
+    set_smem(kern, smem);
+    kern<<<grid, kThreads, smem, st>>>(P, s, cmat, ncols, mid, mid_stride);
+  };
+  // Row counts that are no multiple of 4: windows once the launch is more than
+  // one wave of two CTAs an SM and its loads are what it waits for; a smaller
+  // launch waits for its transforms, and the windows' selects made a lone
+  // query of 19 or 55 rows 1-2 us slower.
+  if (s.other % 4 == 0) run(k_scan_epilogue<Rows::kAligned>);
+  else if (static_cast<uint64_t>(grid.x) * 2 * ncols > 2ull * sm_count()) run(k_scan_epilogue<Rows::kWindow>);
+  else run(k_scan_epilogue<Rows::kScalar>);
   check_launch("k_scan_epilogue");
 }
 

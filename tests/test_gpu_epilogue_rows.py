@@ -30,4 +30,8 @@ def test_row_counts_match_oracle(target, rows):
         got = srv.evaluate_first_dim(srv.expand_query(1, q))
         assert np.array_equal(got.reshape(want.shape), want)
     want = np.stack([ref.make_query(q) for q in qs])
-    assert np.array_equal(srv.make_query_batch([1] * 3, np.stack(qs)), want)
+    # 3: less than a wave of epilogue blocks; 40 and 41: more than one
+    for batch in (3, 40, 41):
+        pick = np.arange(batch) % 3
+        got = srv.make_query_batch([1] * batch, np.stack([qs[i] for i in pick]))
+        assert np.array_equal(got, want[pick]), batch
