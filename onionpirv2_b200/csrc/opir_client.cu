@@ -20,10 +20,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 #include <new>
 #include <stdexcept>
 #include <string>
@@ -640,7 +640,7 @@ struct SecretArgs {
   uint32_t n, cols;
   uint32_t ntile, col_tiles, k_tiles, stages;
   const uint64_t *colsum;
-  volatile uint32_t *err;  // mapped host memory
+  volatile uint32_t *err;
 };
 constexpr int kSecretThreads = 64 + 256;  // producer, MMA issuer, 8 finishing warps
 constexpr uint32_t kMaxSecretStages = 8;
@@ -867,62 +867,6 @@ uint64_t mulmod(uint64_t a, uint64_t b, uint64_t m) {
 
 }  // namespace
 
-namespace {
-
-// Error words of the tensor-core product in one mapped page of pinned host
-// memory per process (the kernels write a word only when a bounded wait runs
-// out, so reading it takes no copy). Pinning memory takes about a millisecond,
-// more than a whole batch, hence one page for all handles: a handle takes a
-// word at its first product and gives it back when it is destroyed, the page
-// goes with the last one. Handles beyond the page's words pin their own.
-class ErrorWords {
- public:
-  uint32_t *take() {
-    std::lock_guard<std::mutex> lock(mu_);
-    if (!page_) {
-      page_ = pin(kWords);
-      for (uint32_t i = kWords; i-- > 0;) free_.push_back(page_ + i);
-    }
-    if (free_.empty()) return pin(1);
-    uint32_t *w = free_.back();
-    free_.pop_back();
-    *w = 0;
-    return w;
-  }
-  void give_back(uint32_t *w) {
-    std::lock_guard<std::mutex> lock(mu_);
-    if (!page_ || w < page_ || w >= page_ + kWords) {
-      cudaFreeHost(w);
-      return;
-    }
-    free_.push_back(w);
-    if (free_.size() == kWords) {
-      free_.clear();
-      cudaFreeHost(page_);
-      page_ = nullptr;
-    }
-  }
-
- private:
-  static constexpr uint32_t kWords = 1024;
-  static uint32_t *pin(uint32_t words) {
-    void *p = nullptr;
-    ck(cudaHostAlloc(&p, words * sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable),
-       "client error word");
-    std::memset(p, 0, words * sizeof(uint32_t));
-    return static_cast<uint32_t *>(p);
-  }
-  std::mutex mu_;
-  uint32_t *page_ = nullptr;
-  std::vector<uint32_t *> free_;
-};
-ErrorWords &error_words() {
-  static ErrorWords *w = new ErrorWords;  // never destroyed: handles may outlive static objects
-  return *w;
-}
-
-}  // namespace
-
 struct opir_client {
   opir_params params{};
   int device = 0;
@@ -935,10 +879,11 @@ struct opir_client {
   DevBuf<int8_t> msgs;       // [1 + h][n]: s, then sigma_{N/2^i + 1}(s) for i < h
   DevBuf<uint64_t> fw;       // [K][n]: forward NTT twiddles per limb
   DevBuf<KeyRow> keyrows;
-  // tensor-core decryption: A = S + 1 (built on first use), per-call scratch
+  // tensor-core product: A = S + 1 and the error word (built on first use),
+  // per-call scratch
   DevBuf<uint8_t> tc_a, tc_q;
   DevBuf<uint64_t> tc_colsum;
-  uint32_t *tc_err = nullptr;        // error word of the product (ErrorWords)
+  DevBuf<uint32_t> tc_err;
   DevBuf<uint64_t> pk_idx;
   uint64_t *idx_staging = nullptr;   // pinned copy of the last call's indices
   size_t idx_staging_cap = 0;
@@ -1220,7 +1165,8 @@ void ensure_secret_matrix(opir_client &c, cudaStream_t st) {
   const uint32_t n = c.n;
   opir::DevBuf<uint8_t> a;
   a.alloc(static_cast<size_t>(n) * n);
-  if (!c.tc_err) c.tc_err = error_words().take();
+  c.tc_err.alloc(1);
+  ck(cudaMemsetAsync(c.tc_err.p, 0, sizeof(uint32_t), st), "client error word");
   k_client_secret_matrix<<<n, kBlock, 0, st>>>(c.msgs.p, n, a.p);
   launched("secret matrix launch");
   std::swap(c.tc_a.p, a.p);
@@ -1253,9 +1199,7 @@ void secret_product(const opir_client &c, uint64_t cols, const uint8_t *planes,
   const size_t stage = 16384 + NP * a.ntile * 128;
   a.stages = static_cast<uint32_t>(std::min<size_t>(kMaxSecretStages, (kLimit - 1024 - 256) / stage));
   a.colsum = colsum;
-  void *err = nullptr;
-  ck(cudaHostGetDevicePointer(&err, c.tc_err, 0), "client error word");
-  a.err = static_cast<volatile uint32_t *>(err);
+  a.err = c.tc_err.p;
   CUtensorMap map_a, map_x;
   opir::make_plane_map(&map_a, c.tc_a.p, n, n, 1, 128, 128);
   opir::make_plane_map(&map_x, planes, n, cols, NP, a.ntile, 128);
@@ -1267,13 +1211,24 @@ void secret_product(const opir_client &c, uint64_t cols, const uint8_t *planes,
   launched("client secret product launch");
 }
 
-// Synchronises the stream and reads the products' error word, which lies in
-// mapped host memory: the kernels write it only when a bounded wait runs out.
-void check_product_error(opir_client &c, cudaStream_t st, const char *what) {
+// Synchronises the stream and reports a product whose bounded wait ran out. A
+// wait runs out after kWaitCycles SM cycles, so a call that is back sooner than
+// these take at 8 GHz, four times the clock, cannot have set the error word,
+// and only a later one reads it. The read would add 9 us to every call of 38;
+// the word in mapped host memory took no read, but pinning it and giving it
+// back took 2.9 ms a client (created, one batch of 64, destroyed: 3.6 ms).
+using Clock = std::chrono::steady_clock;
+constexpr std::chrono::nanoseconds kReadErrorAfter{opir::tc::kWaitCycles / 8};
+void check_product_error(const opir_client &c, cudaStream_t st, Clock::time_point begin,
+                         const char *what) {
   ck(cudaStreamSynchronize(st), what);
-  const uint32_t err = *const_cast<volatile uint32_t *>(c.tc_err);
+  if (Clock::now() - begin < kReadErrorAfter) return;
+  uint32_t err = 0;
+  ck(cudaMemcpyAsync(&err, c.tc_err.p, sizeof(err), cudaMemcpyDeviceToHost, st), what);
+  ck(cudaStreamSynchronize(st), what);
   if (err) {
-    *c.tc_err = 0;
+    ck(cudaMemsetAsync(c.tc_err.p, 0, sizeof(err), st), what);
+    ck(cudaStreamSynchronize(st), what);
     throw std::runtime_error(std::string(what) + ": tensor-core product gave up (error bits " +
                              std::to_string(err) + ")");
   }
@@ -1293,6 +1248,7 @@ void launch_pack_tc(uint64_t n_q, const uint64_t *pt_idx, cudaStream_t st, const
   const uint32_t n = c.n, limbs = c.limbs;
   const opir_params &p = c.params;
   if (p.l_ep > 16) throw std::runtime_error("client pack: L_EP above 16");
+  const Clock::time_point begin = Clock::now();
   ensure_secret_matrix(c, st);
   const uint64_t cols = n_q * limbs;  // one column per query and limb
   ensure_planes(c, 8, cols, st);
@@ -1339,7 +1295,7 @@ void launch_pack_tc(uint64_t n_q, const uint64_t *pt_idx, cudaStream_t st, const
   k_client_pack_constants<<<static_cast<unsigned>(n_q), 128, 0, st>>>(c.pk_idx.p, L, n, limbs,
                                                                      c.mods[0], c.mods[1], out);
   launched("client constants launch");
-  check_product_error(c, st, "client pack");
+  check_product_error(c, st, begin, "client pack");
 }
 
 // Plane counts of a reduced response: 3 (narrow moduli, small_q below 2^24), 4
@@ -1347,6 +1303,7 @@ void launch_pack_tc(uint64_t n_q, const uint64_t *pt_idx, cudaStream_t st, const
 void launch_decrypt_tc(uint64_t n_resp, cudaStream_t st, const uint64_t *resp, opir_client &c,
                        uint64_t *pt, unsigned long long *noise) {
   const uint32_t n = c.n, nr = static_cast<uint32_t>(n_resp);
+  const Clock::time_point begin = Clock::now();
   ensure_secret_matrix(c, st);
   FinishDecrypt fin{};
   fin.resp = resp;
@@ -1368,7 +1325,7 @@ void launch_decrypt_tc(uint64_t n_resp, cudaStream_t st, const uint64_t *resp, o
   if (fin.dc.narrow) run(std::integral_constant<int, 3>{});
   else if (sq < (1ull << 29)) run(std::integral_constant<int, 4>{});
   else run(std::integral_constant<int, 7>{});
-  check_product_error(c, st, "client decrypt");
+  check_product_error(c, st, begin, "client decrypt");
 }
 
 void launch_decrypt(uint64_t n_resp, cudaStream_t st, const uint64_t *resp, const opir_client &c,
@@ -1616,7 +1573,7 @@ void opir_client_destroy(opir_client *c) {
     c->tc_a.reset();
     c->tc_q.reset();
     c->tc_colsum.reset();
-    if (c->tc_err) error_words().give_back(c->tc_err);
+    c->tc_err.reset();
     c->pk_idx.reset();
     if (c->idx_staging) cudaFreeHost(c->idx_staging);
     c->consts.reset();
