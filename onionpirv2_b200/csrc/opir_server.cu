@@ -157,8 +157,9 @@ struct opir_tree {
   DevBuf<uint64_t> out;            // (L + 1) x 2N u64
   cudaEvent_t q_done = nullptr, first_done = nullptr;
   std::vector<cudaEvent_t> done;   // per level
-  // short first dimensions (n0 <= kMaxRowsN0): every level's rows, answered in
-  // one launch, and every level's selected ciphertext
+  // short first dimensions of trees that are not tall (first_dim_by_rows):
+  // every level's rows, answered in one launch, and every level's selected
+  // ciphertext
   DevBuf<opir::FirstDimRow> rows;
   DevBuf<const uint32_t *> selected;
   std::string last_error;
@@ -918,6 +919,23 @@ void combine_k1(opir_server *s, uint32_t n, const uint64_t *d_partials, uint64_t
                            n, s->stream);
   opir::launch_modswitch(s->dp, s->comb[cur].p, G, d_resp, nullptr, resp_bytes_of(s->params), n,
                          s->stream);
+}
+
+// Whether a tree's first dimension goes row by row (tree_query_rows) or through
+// a scan a level. A scan costs about the same for 8 columns as for 64, a row its
+// n0 products and two reads at a level stride that grows with the rows, so the
+// line falls as n0p^2. Milliseconds a query, rows / scan, by the rows of the
+// largest level (half of all):
+//   n0 <= 8:  8192   8.3-8.6 / 10.4-10.5     16384   20.2-20.6 / 18.9-19.0
+//   n0 = 32:  2048   3.50 / 3.91               512   1.28 / 2.39
+//   n0 = 64:   512   2.37 / 2.47              1024   4.29 / 3.02
+bool first_dim_by_rows(const std::vector<opir_server *> &levels) {
+  constexpr uint64_t kMaxRowsWork = 1ull << 21;  // rows n0p^2
+  for (const opir_server *l : levels)
+    if (l->shape.n0p > opir::kMaxRowsN0 ||
+        static_cast<uint64_t>(l->shape.other) * l->shape.n0p * l->shape.n0p > kMaxRowsWork)
+      return false;
+  return true;
 }
 
 // opir_tree_query over short first dimensions, from the query's ciphertext in
@@ -2095,7 +2113,7 @@ opir_status opir_tree_create(const opir_params *scheme, const opir_tree_params *
       ensure_capacity(t->q, 1);
       grow_keyptr_slots(t->q, 2);
       for (opir_server *l : t->levels) ensure_capacity(l, 1);
-      if (t->q->shape.n0 <= opir::kMaxRowsN0) {
+      if (first_dim_by_rows(t->levels)) {
         std::vector<opir::FirstDimRow> rows;
         std::vector<const uint32_t *> selected;
         for (opir_server *l : t->levels) {
