@@ -579,7 +579,7 @@ struct FinishDecrypt {  // pt = round(phase t / sq) and the response's max noise
   unsigned long long *noise;
   DecConst dc;
   BigMod mod;     // sq (seven planes)
-  uint64_t bias;  // the multiple 2 n + 1 of sq: |x s| <= n sq
+  uint64_t bias;  // the multiple 2 n + 1 of sq (three planes): |x s| <= n sq
   uint32_t n;
   __device__ __forceinline__ uint64_t operand(uint32_t c, uint32_t i) const {
     return __ldg(resp + static_cast<uint64_t>(c) * (2 * n) + i);
@@ -587,17 +587,16 @@ struct FinishDecrypt {  // pt = round(phase t / sq) and the response's max noise
   template <int NP>
   __device__ __forceinline__ uint64_t compute(uint32_t, int64_t lo, int64_t hi, uint64_t c0,
                                               uint64_t &worst) const {
-    const uint64_t v = static_cast<uint64_t>(lo) + bias;  // NP <= 4: below 2^38 (narrow), 2^43
     if (NP == 3) {
+      const uint64_t v = static_cast<uint64_t>(lo) + bias;  // below 2^38
       const uint32_t sq = static_cast<uint32_t>(dc.sq);
       uint32_t w = 0;
       const uint32_t m = decrypt_narrow(static_cast<uint32_t>(v) - div_narrow(v, sq, dc.m_sq) * sq, c0, dc, w);
       worst = w;
       return m;
     }
-    const uint64_t prod = NP <= 4 ? v - div_barrett(v, dc.sq, dc.mu_sq) * dc.sq : mod(lo, hi);
     worst = 0;
-    return decrypt_coeff(prod, c0, dc, worst);
+    return decrypt_coeff(mod(lo, hi), c0, dc, worst);
   }
   template <int NP>
   __device__ __forceinline__ void store(uint32_t c, uint32_t i, uint64_t v, uint64_t worst) const {
@@ -1138,6 +1137,8 @@ BigMod big_mod(uint64_t q, uint32_t n, uint32_t lo_bits, uint32_t hi_bits) {
   // hi' + lo' / 2^32 < 2^(hi_bits + ln + 2) + 2^(lo_bits + ln + 2 - 32)
   const uint32_t top = std::max(hi_bits + ln + 3, lo_bits + ln + 3 > 32 ? lo_bits + ln + 3 - 32 : 1);
   b.sh = top > 32 ? top - 32 : 0;
+  // the estimate's error and m in 32 bits both need q above 2^(32 + sh)
+  if (q <= 1ull << (32 + b.sh)) throw std::invalid_argument("client product: modulus too small");
   b.m = static_cast<uint32_t>((static_cast<u128>(1) << (64 + b.sh)) / q);
   // the least multiple of q at or above the magnitude of both parts, split
   // with lb >= 2 n 2^lo_bits
@@ -1298,8 +1299,8 @@ void launch_pack_tc(uint64_t n_q, const uint64_t *pt_idx, cudaStream_t st, const
   check_product_error(c, st, begin, "client pack");
 }
 
-// Plane counts of a reduced response: 3 (narrow moduli, small_q below 2^24), 4
-// (below 2^29) or 7 (below 2^50).
+// Plane counts of a reduced response: 3 (narrow moduli: CONFIG_N2048_K1_COMP's
+// 22 bits) or 7 (up to 2^50: CONFIG_N4096_K2_MP's).
 void launch_decrypt_tc(uint64_t n_resp, cudaStream_t st, const uint64_t *resp, opir_client &c,
                        uint64_t *pt, unsigned long long *noise) {
   const uint32_t n = c.n, nr = static_cast<uint32_t>(n_resp);
@@ -1323,7 +1324,6 @@ void launch_decrypt_tc(uint64_t n_resp, cudaStream_t st, const uint64_t *resp, o
     secret_product<NP>(c, n_resp, c.tc_q.p, c.tc_colsum.p, fin, st);
   };
   if (fin.dc.narrow) run(std::integral_constant<int, 3>{});
-  else if (sq < (1ull << 29)) run(std::integral_constant<int, 4>{});
   else run(std::integral_constant<int, 7>{});
   check_product_error(c, st, begin, "client decrypt");
 }
