@@ -1137,8 +1137,10 @@ BigMod big_mod(uint64_t q, uint32_t n, uint32_t lo_bits, uint32_t hi_bits) {
   // hi' + lo' / 2^32 < 2^(hi_bits + ln + 2) + 2^(lo_bits + ln + 2 - 32)
   const uint32_t top = std::max(hi_bits + ln + 3, lo_bits + ln + 3 > 32 ? lo_bits + ln + 3 - 32 : 1);
   b.sh = top > 32 ? top - 32 : 0;
-  // the estimate's error and m in 32 bits both need q above 2^(32 + sh)
-  if (q <= 1ull << (32 + b.sh)) throw std::invalid_argument("client product: modulus too small");
+  // the estimate's error and m in 32 bits both need q above 2^(32 + sh), the
+  // remainder 3 q in a word
+  if (q <= 1ull << (32 + b.sh) || q >> 62)
+    throw std::invalid_argument("client product: modulus out of range");
   b.m = static_cast<uint32_t>((static_cast<u128>(1) << (64 + b.sh)) / q);
   // the least multiple of q at or above the magnitude of both parts, split
   // with lb >= 2 n 2^lo_bits
@@ -1152,13 +1154,9 @@ BigMod big_mod(uint64_t q, uint32_t n, uint32_t lo_bits, uint32_t hi_bits) {
 // The tensor-core form serves decryption and packing batches of at least
 // kTcMinResponses (OPIR_CLIENT_TC=0 turns it off).
 constexpr uint64_t kTcMinResponses = 32;
-// any_limbs: decryption, whose modulus (small_q) is one prime for both sets.
-bool tc_enabled(const opir_client &c, uint64_t items, uint64_t modulus_bound,
-                bool any_limbs = false) {
+bool tc_enabled(uint64_t items) {
   const char *v = std::getenv("OPIR_CLIENT_TC");
-  if ((v && v[0] == '0') || !window_enabled()) return false;
-  return (any_limbs || c.limbs == 1) && c.n % 128 == 0 && c.n <= 8192 &&
-         modulus_bound < (1ull << 29) && items >= kTcMinResponses;
+  return !(v && v[0] == '0') && window_enabled() && items >= kTcMinResponses;
 }
 
 void ensure_secret_matrix(opir_client &c, cudaStream_t st) {
@@ -1317,7 +1315,10 @@ void launch_decrypt_tc(uint64_t n_resp, cudaStream_t st, const uint64_t *resp, o
   const auto run = [&](auto np) {
     constexpr int NP = decltype(np)::value;
     ensure_planes(c, NP, n_resp, st);
-    if (NP > 4) fin.mod = big_mod(sq, n, 32, 18);  // sq < 2^50
+    if (NP > 4) {
+      if (sq >> 50) throw std::invalid_argument("client product: small_q above 50 bits");
+      fin.mod = big_mod(sq, n, 32, 18);
+    }
     k_client_planes<NP><<<nr, kBlock, 0, st>>>(resp + n, 2ull * n, n, nr, sq, fin.dc.mu_sq, c.tc_q.p,
                                                c.tc_colsum.p, nullptr, 1);
     launched("client planes launch");
@@ -1608,10 +1609,7 @@ opir_status opir_client_generate_queries_device(opir_client *c, uint32_t n,
         throw std::out_of_range("PIR plaintext index exceeds the runtime layout");
     DeviceGuard g(c->device);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const uint64_t qmax = std::max(c->params.q1, c->params.q2);
-    const bool tc = c->limbs == 1 ? tc_enabled(*c, n, qmax)
-                                  : tc_enabled(*c, n, 0, true) && qmax < (1ull << 60);
-    if (tc) {
+    if (tc_enabled(n)) {
       launch_pack_tc(n, pt_idx, st, d_a, d_e, *c, d_queries);
       return;
     }
@@ -1653,8 +1651,7 @@ opir_status opir_client_decrypt_device(opir_client *c, uint32_t n, const uint64_
       ck(cudaMemsetAsync(d_max_noise, 0, static_cast<size_t>(n) * sizeof(uint64_t), st),
          "noise reset");
     auto *noise = reinterpret_cast<unsigned long long *>(d_max_noise);
-    const uint64_t sq = c->params.small_q;
-    if (tc_enabled(*c, n, sq < (1ull << 29) ? sq : 0, true) && sq < (1ull << 50))
+    if (tc_enabled(n))
       launch_decrypt_tc(n, st, d_responses, *c, d_plaintexts, noise);
     else
       launch_decrypt(n, st, d_responses, *c, d_plaintexts, noise);
