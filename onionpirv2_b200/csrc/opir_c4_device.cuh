@@ -46,11 +46,6 @@ __device__ __forceinline__ int posB(int t, int k) { return ((t >> 6) << 9) + (t 
 __device__ __forceinline__ int posC(int t, int k) { return ((t >> 3) << 6) + (t & 7) + 8 * k; }
 __device__ __forceinline__ int posD(int t, int k) { return 8 * t + k; }
 
-// a w mod q in [0, 2q) for any 64-bit a (Shoup; ws = floor(w 2^64 / q))
-template <uint64_t Q>
-__device__ __forceinline__ uint64_t mul_shoup(uint64_t a, uint64_t w, uint64_t ws) {
-  return a * w - __umul64hi(a, ws) * Q;
-}
 template <uint64_t Q>
 __device__ __forceinline__ uint64_t add_mod(uint64_t a, uint64_t b) {
   const uint64_t s = a + b;
@@ -64,22 +59,6 @@ __device__ __forceinline__ uint64_t sub_mod(uint64_t a, uint64_t b) {
 template <uint64_t Q>
 __device__ __forceinline__ uint64_t neg_mod(uint64_t a) {
   return a ? Q - a : 0;
-}
-
-// x mod q for x < 2^126: x = h 2^64 + l, h 2^64 mod q by Shoup with
-// c = 2^64 mod q, l mod q by a 64-bit Barrett estimate.
-template <uint64_t Q>
-__device__ __forceinline__ uint64_t red128(unsigned __int128 x) {
-  constexpr uint64_t c = static_cast<uint64_t>((static_cast<unsigned __int128>(1) << 64) % Q);
-  constexpr uint64_t cs = static_cast<uint64_t>((static_cast<unsigned __int128>(c) << 64) / Q);
-  constexpr uint64_t mu = ~0ull / Q;  // floor(2^64 / q)
-  const uint64_t h = static_cast<uint64_t>(x >> 64), l = static_cast<uint64_t>(x);
-  const uint64_t r1 = mul_shoup<Q>(h, c, cs);            // [0, 2q)
-  const uint64_t r2 = l - __umul64hi(l, mu) * Q;          // [0, 3q)
-  uint64_t r = r1 + r2;                                   // [0, 5q) < 2^63
-  r = min(r, r - 4 * Q);
-  r = min(r, r - 2 * Q);
-  return min(r, r - Q);
 }
 
 // ----------------------------------------------------------------- NTT

@@ -354,19 +354,15 @@ LimbTables64 make_limb_tables64(uint32_t n, uint64_t q, uint64_t root) {
     pw[i] = static_cast<uint64_t>(static_cast<u128>(pw[i - 1]) * root % q);
     ipw[i] = static_cast<uint64_t>(static_cast<u128>(ipw[i - 1]) * rinv % q);
   }
-  auto shoup = [q](uint64_t w) { return static_cast<uint64_t>((static_cast<u128>(w) << 64) / q); };
-  t.fw.resize(n); t.fw_sh.resize(n); t.iw.resize(n); t.iw_sh.resize(n);
+  t.fw.resize(n);
+  t.iw.resize(n);
   for (uint32_t k = 0; k < n; ++k) {
     const uint32_t e = bitrev(k, lg);
-    t.fw[k] = pw[e]; t.fw_sh[k] = shoup(pw[e]);
-    t.iw[k] = ipw[e]; t.iw_sh[k] = shoup(ipw[e]);
+    t.fw[k] = pw[e];
+    t.iw[k] = ipw[e];
   }
-  uint64_t ninv = 0;
-  invert_mod(n % q, q, ninv);
-  t.n_inv = ninv;
-  t.n_inv_sh = shoup(ninv);
-  t.w1_ninv = static_cast<uint64_t>(static_cast<u128>(t.iw[1]) * ninv % q);
-  t.w1_ninv_sh = shoup(t.w1_ninv);
+  invert_mod(n % q, q, t.n_inv);
+  t.w1_ninv = static_cast<uint64_t>(static_cast<u128>(t.iw[1]) * t.n_inv % q);
   return t;
 }
 

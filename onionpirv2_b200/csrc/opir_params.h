@@ -38,11 +38,10 @@ opir_params derive_params_k2mp(const opir_layout &layout);
 // PirParams under CONFIG_N2048_K1 (one 60-bit prime at N = 2048; q1 = q2 = 0).
 opir_params derive_params_k1p(const opir_layout &layout);
 
-// 64-bit limb tables: bit-reversed powers with Shoup companions
-// floor(w 2^64 / q), N^-1 and iw[1] N^-1 with theirs.
+// 64-bit limb tables: bit-reversed powers, N^-1 and iw[1] N^-1.
 struct LimbTables64 {
-  uint64_t q = 0, n_inv = 0, n_inv_sh = 0, w1_ninv = 0, w1_ninv_sh = 0;
-  std::vector<uint64_t> fw, fw_sh, iw, iw_sh;
+  uint64_t q = 0, n_inv = 0, w1_ninv = 0;
+  std::vector<uint64_t> fw, iw;
 };
 LimbTables64 make_limb_tables64(uint32_t n, uint64_t q, uint64_t root);
 
