@@ -9,14 +9,13 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <set>
 #include <stdexcept>
 #include <string>
-#include <utility>
 
 #include "opir_c4_device.cuh"
+#include "opir_launch.h"
 
 #include <cooperative_groups.h>
 
@@ -24,6 +23,9 @@ namespace opir4 {
 
 namespace {
 
+using opir::launch_cluster;
+using opir::set_smem;
+using opir::sm_count;
 using u128 = unsigned __int128;
 using i128 = __int128;
 
@@ -44,62 +46,6 @@ void check_launch(const char *what) {
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
-}
-
-// SMs of the current device (cached per device).
-int sm_count() {
-  static std::mutex mu;
-  static std::map<int, int> cache;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find(dev);
-  if (it != cache.end()) return it->second;
-  int n = 0;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
-    cudaGetLastError();
-    n = 148;
-  }
-  cache[dev] = n;
-  return n;
-}
-
-// Launch with a 1-D cluster of `c` CTAs along x.
-template <typename Kern, typename... Args>
-void launch_cluster(Kern kernel, int c, dim3 grid, size_t smem, cudaStream_t st, const char *what,
-                    Args... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = c;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
-  if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
-  check_launch(what);
-}
-
-template <typename K>
-void set_smem(K kernel, size_t bytes) {
-  static std::mutex mu;
-  static std::map<std::pair<int, const void *>, size_t> granted;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const auto key = std::make_pair(dev, reinterpret_cast<const void *>(kernel));
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = granted.find(key);
-  if (it != granted.end() && it->second >= bytes) return;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(bytes));
-  if (e != cudaSuccess)
-    throw std::runtime_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-  granted[key] = bytes;
 }
 
 constexpr size_t plane_bytes(int np) { return static_cast<size_t>(np) * kPad * sizeof(uint64_t); }
@@ -1189,19 +1135,16 @@ void launch_expand_level(const Dev4 &P, const Shape4 &s, uint32_t d, const uint6
     return;
   }
   const dim3 grid(nodes * split, 2, batch);
-  if (split == 8) {
-    set_smem(k4_expand_level_split<8>, smem);
-    launch_cluster(k4_expand_level_split<8>, 8, grid, smem, st, "k4_expand_level_split", P, inv, k,
-                   in, in_stride, out, out_stride, bv_keys, koff);
-  } else if (split == 4) {
-    set_smem(k4_expand_level_split<4>, smem);
-    launch_cluster(k4_expand_level_split<4>, 4, grid, smem, st, "k4_expand_level_split", P, inv, k,
-                   in, in_stride, out, out_stride, bv_keys, koff);
-  } else {
-    set_smem(k4_expand_level_split<2>, smem);
-    launch_cluster(k4_expand_level_split<2>, 2, grid, smem, st, "k4_expand_level_split", P, inv, k,
-                   in, in_stride, out, out_stride, bv_keys, koff);
-  }
+  if (split == 8)
+    launch_cluster(k4_expand_level_split<8>, 8, grid, kThreads, smem, st, "k4_expand_level_split", P,
+                   inv, k, in, in_stride, out, out_stride, bv_keys, koff);
+  else if (split == 4)
+    launch_cluster(k4_expand_level_split<4>, 4, grid, kThreads, smem, st, "k4_expand_level_split", P,
+                   inv, k, in, in_stride, out, out_stride, bv_keys, koff);
+  else
+    launch_cluster(k4_expand_level_split<2>, 2, grid, kThreads, smem, st, "k4_expand_level_split", P,
+                   inv, k, in, in_stride, out, out_stride, bv_keys, koff);
+  check_launch("k4_expand_level_split");
 }
 
 void launch_selectors(const Dev4 &P, const Shape4 &s, const uint64_t *leaves, uint64_t leaf_stride,
@@ -1286,15 +1229,13 @@ void launch_mux_level(const Dev4 &P, const Shape4 &s, uint32_t level, uint32_t t
     // offset == extra == 0 here, so level 0 pairs (2i, 2i + 1) into i
     const uint32_t xs = level == 0 ? 2 : 1, yoff = level == 0 ? 1 : half;
     const dim3 g(n_pairs * split, 2, batch);
-    if (split == 4) {
-      set_smem(k4_mux_level_split<4>, smem);
-      launch_cluster(k4_mux_level_split<4>, 4, g, smem, st, "k4_mux_level_split", P, s, level, xs,
-                     yoff, in, out, mid_stride, sel);
-    } else {
-      set_smem(k4_mux_level_split<2>, smem);
-      launch_cluster(k4_mux_level_split<2>, 2, g, smem, st, "k4_mux_level_split", P, s, level, xs,
-                     yoff, in, out, mid_stride, sel);
-    }
+    if (split == 4)
+      launch_cluster(k4_mux_level_split<4>, 4, g, kThreads, smem, st, "k4_mux_level_split", P, s,
+                     level, xs, yoff, in, out, mid_stride, sel);
+    else
+      launch_cluster(k4_mux_level_split<2>, 2, g, kThreads, smem, st, "k4_mux_level_split", P, s,
+                     level, xs, yoff, in, out, mid_stride, sel);
+    check_launch("k4_mux_level_split");
     return;
   }
   set_smem(k4_mux_level, smem);

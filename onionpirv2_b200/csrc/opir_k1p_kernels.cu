@@ -12,8 +12,8 @@
 #include "opir_k1p_kernels.h"
 
 #include "opir_fold60.cuh"
+#include "opir_launch.h"
 
-#include <map>
 #include <mutex>
 #include <set>
 #include <stdexcept>
@@ -25,6 +25,9 @@ namespace opir1 {
 
 namespace {
 
+using opir::launch_cluster;
+using opir::set_smem;
+using opir::sm_count;
 using u128 = unsigned __int128;
 
 constexpr int kThreads = 256;
@@ -43,42 +46,7 @@ void check_launch(const char *what) {
   opir4::note_launches(1);
 }
 
-template <typename K>
-void set_smem(K kernel, size_t bytes) {
-  static std::mutex mu;
-  static std::map<std::pair<int, const void *>, size_t> granted;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const auto key = std::make_pair(dev, reinterpret_cast<const void *>(kernel));
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = granted.find(key);
-  if (it != granted.end() && it->second >= bytes) return;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(bytes));
-  if (e != cudaSuccess)
-    throw std::runtime_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-  granted[key] = bytes;
-}
-
 constexpr size_t plane_bytes(int np) { return static_cast<size_t>(np) * kPad * sizeof(uint64_t); }
-
-// SMs of the current device (cached per device).
-int sms() {
-  static std::mutex mu;
-  static std::map<int, int> cache;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find(dev);
-  if (it != cache.end()) return it->second;
-  int n = 0;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
-    cudaGetLastError();
-    n = 1;
-  }
-  cache[dev] = n;
-  return n;
-}
 
 // ------------------------------------------------------------ arithmetic
 __device__ __forceinline__ uint64_t mix64(uint64_t z) {  // splitmix64 finaliser
@@ -1098,30 +1066,10 @@ namespace {
 int split_of(uint64_t ctas, int widest) {
   if (!opir4::split_enabled()) return 1;
   int c = widest;
-  while (c > 1 && c * ctas > 2ull * sms()) c /= 2;
+  while (c > 1 && c * ctas > 2ull * sm_count()) c /= 2;
   return c;
 }
 
-template <typename Kern, typename... Args>
-void launch_cluster(Kern kernel, int c, dim3 grid, size_t smem, cudaStream_t st, const char *what,
-                    Args... args) {
-  set_smem(kernel, smem);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = c;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
-  if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
-  check_launch(what);
-}
 }  // namespace
 
 void launch_expand_level(const Dev1 &P, const Shape1 &s, uint32_t d, const uint64_t *in,
@@ -1140,7 +1088,7 @@ void launch_expand_level(const Dev1 &P, const Shape1 &s, uint32_t d, const uint6
     throw std::invalid_argument("NTT-form children only at the last expansion level");
   if (ntt_nodes > 0) {
     const dim3 grid(ntt_nodes, 1, batch);
-    if (static_cast<uint64_t>(ntt_nodes) * batch > static_cast<uint64_t>(sms())) {
+    if (static_cast<uint64_t>(ntt_nodes) * batch > static_cast<uint64_t>(sm_count())) {
       set_smem(k1p_expand_level_ntt<2>, smem);
       k1p_expand_level_ntt<2><<<grid, kThreads, smem, st>>>(P, galois, galois_inv, k, in,
                                                              in_stride, out, out_stride, bv_keys,
@@ -1160,18 +1108,19 @@ void launch_expand_level(const Dev1 &P, const Shape1 &s, uint32_t d, const uint6
   if (split > 1) {
     const dim3 g(rest * split, 1, batch);
     if (split == 8)
-      launch_cluster(k1p_expand_level_split<8>, 8, g, smem, st, "k1p_expand_level_split", P, galois_inv, k,
-                     in, in_stride, out, out_stride, bv_keys, koff);
+      launch_cluster(k1p_expand_level_split<8>, 8, g, kThreads, smem, st, "k1p_expand_level_split", P,
+                     galois_inv, k, in, in_stride, out, out_stride, bv_keys, koff);
     else if (split == 4)
-      launch_cluster(k1p_expand_level_split<4>, 4, g, smem, st, "k1p_expand_level_split", P, galois_inv, k,
-                     in, in_stride, out, out_stride, bv_keys, koff);
+      launch_cluster(k1p_expand_level_split<4>, 4, g, kThreads, smem, st, "k1p_expand_level_split", P,
+                     galois_inv, k, in, in_stride, out, out_stride, bv_keys, koff);
     else
-      launch_cluster(k1p_expand_level_split<2>, 2, g, smem, st, "k1p_expand_level_split", P, galois_inv, k,
-                     in, in_stride, out, out_stride, bv_keys, koff);
+      launch_cluster(k1p_expand_level_split<2>, 2, g, kThreads, smem, st, "k1p_expand_level_split", P,
+                     galois_inv, k, in, in_stride, out, out_stride, bv_keys, koff);
+    check_launch("k1p_expand_level_split");
     return;
   }
   const dim3 grid(rest, 1, batch);
-  if (ctas > static_cast<uint64_t>(sms())) {
+  if (ctas > static_cast<uint64_t>(sm_count())) {
     set_smem(k1p_expand_level<2>, smem);
     k1p_expand_level<2><<<grid, kThreads, smem, st>>>(P, galois_inv, k, in, in_stride, out,
                                                        out_stride, bv_keys, koff, ntt_nodes);
@@ -1190,7 +1139,7 @@ void launch_selectors(const Dev1 &P, const Shape1 &s, const uint64_t *leaves, ui
   const size_t smem = plane_bytes(kGroup);
   const uint32_t rows = (s.num_dims - 1) * s.l_ep;
   const dim3 grid(rows, 1, batch);
-  if (static_cast<uint64_t>(rows) * batch >= 2ull * sms()) {
+  if (static_cast<uint64_t>(rows) * batch >= 2ull * sm_count()) {
     set_smem(k1p_selectors<2>, smem);
     k1p_selectors<2><<<grid, kThreads, smem, st>>>(P, s, leaves, leaf_stride, gsw_keys, sel);
   } else {
@@ -1268,11 +1217,12 @@ void launch_mux_level(const Dev1 &P, const Shape1 &s, uint32_t level, uint32_t t
     const uint32_t xs = level == 0 ? 2 : 1, yoff = level == 0 ? 1 : half;
     const dim3 g(n_pairs * split, 1, batch);
     if (split == 4)
-      launch_cluster(k1p_mux_level_split<4>, 4, g, smem, st, "k1p_mux_level_split", P, s, level, xs, yoff,
-                     in, out, mid_stride, sel);
+      launch_cluster(k1p_mux_level_split<4>, 4, g, kThreads, smem, st, "k1p_mux_level_split", P, s,
+                     level, xs, yoff, in, out, mid_stride, sel);
     else
-      launch_cluster(k1p_mux_level_split<2>, 2, g, smem, st, "k1p_mux_level_split", P, s, level, xs, yoff,
-                     in, out, mid_stride, sel);
+      launch_cluster(k1p_mux_level_split<2>, 2, g, kThreads, smem, st, "k1p_mux_level_split", P, s,
+                     level, xs, yoff, in, out, mid_stride, sel);
+    check_launch("k1p_mux_level_split");
     return;
   }
   set_smem(k1p_mux_level, smem);

@@ -4,6 +4,7 @@
 // opir_device.cuh. Thread t owns coefficient positions t + 256 s, s < 8, for
 // every per-coefficient step, so global reads of planes are coalesced.
 #include "opir_kernels.h"
+#include "opir_launch.h"
 #include "opir_ntt.cuh"
 
 #include <cooperative_groups.h>
@@ -12,12 +13,10 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <set>
 #include <stdexcept>
 #include <string>
-#include <utility>
 
 namespace opir {
 
@@ -40,24 +39,6 @@ void check_launch(const char *what) {
     throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// SMs of the current device (cached per device).
-int sm_count() {
-  static std::mutex mu;
-  static std::map<int, int> cache;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = cache.find(dev);
-  if (it != cache.end()) return it->second;
-  int n = 0;
-  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
-    cudaGetLastError();
-    n = 148;
-  }
-  cache[dev] = n;
-  return n;
-}
-
 // Cluster-split MUX levels (k_mux_level_split): on unless OPIR_SPLIT=0.
 bool split_enabled() {
   static const bool on = [] {
@@ -65,25 +46,6 @@ bool split_enabled() {
     return !(e && std::strcmp(e, "0") == 0);
   }();
   return on;
-}
-
-// Raise a kernel's dynamic shared-memory limit once per (device, kernel,
-// size); cudaFuncSetAttribute applies to the current device.
-template <typename K>
-void set_smem(K kernel, size_t bytes) {
-  static std::mutex mu;
-  static std::map<std::pair<int, const void *>, size_t> granted;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const auto key = std::make_pair(dev, reinterpret_cast<const void *>(kernel));
-  std::lock_guard<std::mutex> lock(mu);
-  auto it = granted.find(key);
-  if (it != granted.end() && it->second >= bytes) return;
-  const cudaError_t e = cudaFuncSetAttribute(
-      kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-  if (e != cudaSuccess)
-    throw std::runtime_error(std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
-  granted[key] = bytes;
 }
 
 // ------------------------------------------------------------ split/compose
