@@ -639,7 +639,7 @@ struct SecretArgs {
   uint32_t n, cols;
   uint32_t ntile, col_tiles, k_tiles, stages;
   const uint64_t *colsum;
-  volatile uint32_t *err;
+  uint32_t *err;  // one bit per kind of wait
 };
 constexpr int kSecretThreads = 64 + 256;  // producer, MMA issuer, 8 finishing warps
 constexpr uint32_t kMaxSecretStages = 8;
@@ -652,7 +652,7 @@ constexpr uint32_t kMaxSecretStages = 8;
 // SM's shared memory and TMEM, so that one CTA's set-up and finish run beside
 // another's loop: at 1024 decryptions the loop and set-up take about 17 us
 // alone, the finish 13 (6 of them its DRAM traffic). All waits are bounded; a
-// wait that runs out sets the error word, and the CTA drains its copies and
+// wait that runs out sets its bit of the error word, and the CTA drains its copies and
 // MMAs, frees TMEM and returns.
 template <int NP, class Fin>
 __global__ void __launch_bounds__(kSecretThreads, 2)
@@ -692,7 +692,7 @@ k_client_secret_gemm(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     for (uint32_t kt = 0; kt < a.k_tiles; ++kt) {
       const uint32_t s = kt % a.stages, ph = (kt / a.stages) & 1;
       if (!mbar_wait(&empty[s], ph ^ 1, abort_flag)) {
-        if (lane == 0) { *abort_flag = 1; *a.err = 1u; }
+        if (lane == 0) { *abort_flag = 1; atomicOr(a.err, 1u); }
         break;
       }
       if (lane == 0) {
@@ -710,14 +710,14 @@ k_client_secret_gemm(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
       if (uses == 0) continue;
       const long long t0 = clock64();
       while (!mbar_try(&full[s], (uses - 1) & 1))
-        if (clock64() - t0 > kWaitCycles) { if (lane == 0) *a.err = 8u; break; }
+        if (clock64() - t0 > kWaitCycles) { if (lane == 0) atomicOr(a.err, 8u); break; }
     }
   } else if (warp == 1) {
     const uint32_t idesc = (2u << 4) | ((NP * a.ntile >> 3) << 17) | (8u << 24);  // u8 x u8 -> s32
     for (uint32_t kt = 0; kt < a.k_tiles; ++kt) {
       const uint32_t s = kt % a.stages, ph = (kt / a.stages) & 1;
       if (!mbar_wait(&full[s], ph, abort_flag)) {
-        if (lane == 0) { *abort_flag = 1; *a.err = 2u; }
+        if (lane == 0) { *abort_flag = 1; atomicOr(a.err, 2u); }
         break;
       }
       fence_after();
@@ -734,7 +734,7 @@ k_client_secret_gemm(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     __syncwarp();
     const long long t0 = clock64();
     while (!mbar_try(done, 0))
-      if (clock64() - t0 > kWaitCycles) { if (lane == 0) *a.err = 16u; break; }
+      if (clock64() - t0 > kWaitCycles) { if (lane == 0) atomicOr(a.err, 16u); break; }
   } else {
     const uint32_t quad = warp & 3, part = (warp - 2) >> 2, chunks = a.ntile / 8;
     const uint32_t i = row0 + quad * 32 + lane;
@@ -749,7 +749,7 @@ k_client_secret_gemm(const __grid_constant__ CUtensorMap tm_a, const __grid_cons
     uint64_t next[8];
     load(next, part);
     const bool ok = mbar_wait(done, 0, abort_flag);
-    if (!ok && lane == 0) { *abort_flag = 1; *a.err = 4u; }
+    if (!ok && lane == 0) { *abort_flag = 1; atomicOr(a.err, 4u); }
     fence_after();
     for (uint32_t u = part; ok && u < chunks; u += 2) {
       const uint32_t col0 = ct * a.ntile + 8 * u;
