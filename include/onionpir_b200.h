@@ -585,10 +585,10 @@ opir_status opir_client_generate_queries_device(opir_client *client, uint32_t n,
  *   d_plaintexts : n x N u64 device array, each coefficient below t
  *   d_max_noise  : n u64 device array or NULL: the response's max noise
  *                  |phase - round(small_q m / t)| (client.cpp:389-407)
- * Under CONFIG_N2048_K1_COMP batches of 32 or more run on the tensor cores
- * (as do query batches of 32 or more in opir_client_generate_queries_device);
- * those calls synchronise `stream` before returning, to read the bounded
- * waits' error word of the tensor-core kernel. */
+ * Batches of 32 or more run on the tensor cores under both parameter sets (as
+ * do query batches of 32 or more in opir_client_generate_queries_device);
+ * those calls synchronise `stream` before returning, to report a bounded wait
+ * of the tensor-core kernel that ran out. */
 opir_status opir_client_decrypt_device(opir_client *client, uint32_t n,
                                        const uint64_t *d_responses, uint64_t *d_plaintexts,
                                        uint64_t *d_max_noise, void *stream);

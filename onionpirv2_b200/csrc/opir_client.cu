@@ -12,11 +12,15 @@
 // shared memory; only the epilogue reduces, so the result equals the NTT
 // product mod the same modulus exactly. x is split into parts of at most 31
 // bits so each shared word is an int32 and each partial sum fits an int64.
-// Two forms of the product: the index-list form (list_product: one shared
-// load per nonzero secret coefficient, output and part) for any batch, and
-// for decryption batches that fill the GPU the window form (window_product:
+// Three forms of the product. Batches of kTcMinResponses or more, packing and
+// decryption, run it as one GEMM on the tensor cores: the client's N x N matrix
+// of signed shifts of s by the byte planes of x, an exact integer that the same
+// kernel reduces and finishes (k_client_secret_gemm). Below that, and with
+// OPIR_CLIENT_TC=0, the index-list form (list_product: one shared load per
+// nonzero secret coefficient, output and part) for any batch, and for
+// decryption batches that fill the GPU the window form (window_product:
 // register windows reused across secret coefficients one block apart, int32
-// partial sums). One CTA of kBlock threads per (item, output slice).
+// partial sums), one CTA of kBlock threads per (item, output slice).
 #include <cuda_runtime.h>
 
 #include <algorithm>

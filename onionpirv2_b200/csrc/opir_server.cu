@@ -2221,7 +2221,7 @@ opir_status opir_tree_query(opir_tree *t, uint64_t client_id, const uint64_t *qu
 
 opir_status opir_measure_butterfly_rate(opir_config config, int device, double *per_s) {
   // CONFIG_N2048_K2_MP runs on the residue-pair NTT of CONFIG_N2048_K1_COMP;
-  // CONFIG_N2048_K1 on 64-bit Shoup butterflies like CONFIG_N4096_K2_MP
+  // CONFIG_N2048_K1 on the folding 64-bit butterflies of CONFIG_N4096_K2_MP
   if (!per_s || (config != OPIR_CONFIG_N2048_K1_COMP && config != OPIR_CONFIG_N4096_K2_MP &&
                  config != OPIR_CONFIG_N2048_K2_MP && config != OPIR_CONFIG_N2048_K1))
     return OPIR_ERR_INVALID_ARGUMENT;
